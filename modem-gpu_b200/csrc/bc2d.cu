@@ -13,19 +13,21 @@
 //             column, tridiagonal elimination (the 1-D matrix is diagonally
 //             dominant, so no pivoting is needed);
 //   k_bc_coef the operator coefficients and right-hand side per unknown;
-//   k_bc2d    the 2-D TE system of SetupA_TE / FormAII / MulAibWithXb /
-//             Fwd2DsolveTE (WSfwd2Dmod.f90:32-127, 325-418; FwdTEmod.f90:
-//             104-157): (nh-1)(nz-1) interior nodes, bandwidth m = nz-1.  One
-//             block per slice runs Gaussian elimination on the band with the
-//             right-hand side carried along.  The active (m+1) x (m+1) window
-//             lives in shared memory as a circular buffer; each step writes
-//             the finished row of U out and loads the one new row and column
-//             of A, which no earlier step has touched;
-//   k_bc_back the back substitution, one warp per slice.  The matrix is column diagonally dominant
-//             (the off-diagonal entries are real and sum to minus the real
-//             part of the diagonal), so elimination without row exchanges is
-//             stable; the reference's LAPACK band LU agrees with it to
-//             rounding.
+//   the 2-D TE system of SetupA_TE / FormAII / MulAibWithXb / Fwd2DsolveTE
+//             (WSfwd2Dmod.f90:32-127, 325-418; FwdTEmod.f90:104-157):
+//             (nh-1)(nz-1) interior nodes, complex symmetric and column
+//             diagonally dominant (the off-diagonal entries are real and sum
+//             to minus the real part of the diagonal), so elimination without
+//             row exchanges is stable; the reference's LAPACK band LU agrees
+//             with it to rounding.  In one of two ways:
+//   k_bc_sweep, k_bc_subst   when the shorter axis of the slices has at most
+//             kBcMaxM interior nodes: block elimination of the grid's lines
+//             with the running Schur complement held in registers;
+//   k_bc2d, k_bc_back   longer slices: band elimination with the active
+//             (m+1) x (m+1) window, m = nz-1, in shared memory or, where it
+//             does not fit, in global memory as a circular buffer; each step
+//             writes the finished row of U out and loads the one new row and
+//             column of A, which no earlier step has touched.
 // The output is the full edge vector E0 with the tangential field of the
 // bottom face zero (boundary_ws.f90:155-156): its boundary entries are the
 // BC, its interior entries the first guess.
@@ -207,23 +209,428 @@ struct Op2d {
 }  // namespace
 
 // Coefficients of the 2-D operators and right-hand sides of the slices of a
-// launch chunk, one thread per unknown: the diagonal, A(r, r+1), A(r, r+m)
-// and -A_ib x_b, so that the elimination reads them instead of forming them
-// on its critical path.
+// launch chunk, one thread per unknown: the diagonal, the couplings to the
+// next unknown of its line and to the same unknown of the next line, and
+// -A_ib x_b, so that the elimination reads them instead of forming them on its
+// critical path.  Lines are the slice's columns (unknown iz of column iy at
+// iy m + iz) or, with a.rows, its rows.
 __global__ void k_bc_coef(BcArgs a, int nslices)
 {
     const int m = a.nz - 1, n = (a.nh - 1) * m;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)nslices * n) return;
-    const int q = (int)(t / n), r = (int)(t % n), s = a.slice0 + q;
+    const int q = (int)(t / n), u = (int)(t % n), s = a.slice0 + q;
     const Slice sl(a, s);
     const Op2d op(a, sl);
+    const int nl = a.nh - 1;  // unknowns of a row
+    const int r = a.rows ? (u % nl) * m + u / nl : u;
     const double2 *left = a.side + (size_t)s * 2 * (a.nz + 1), *right = left + (a.nz + 1);
     const double2 *bottom = a.bottom + (size_t)s * (a.nh + 1);
     a.cd[t] = op.diag(r);
-    a.czc[t] = op.zc(r);
-    a.cyc[t] = op.yc(r);
+    a.czc[t] = a.rows ? op.yc(r) : op.zc(r);
+    a.cyc[t] = a.rows ? op.zc(r) : op.yc(r);
     a.cb[t] = op.rhs(r, left, right, bottom);
+}
+
+// ---------------------------------------------------------------------------
+// Block elimination of one slice.  The unknowns are n lines of m (m the
+// shorter way); line q couples to line q + 1 through the diagonal matrix C_q
+// (real), so eliminating the lines from one end leaves the Schur complements
+//   S_q = D_q - C_{q-1} S_{q-1}^-1 C_{q-1},  f_q = b_q - C_{q-1} y_{q-1},
+//   y_q = S_q^-1 f_q.
+// Both ends are eliminated at once, by two thread blocks that meet in the
+// middle line, which halves the serial chain and gives twice the blocks; then
+// x_q = y_q - S_q^-1 C x_{q+1} outwards from the middle.
+//
+// S stays complex symmetric, so a block holds its lower triangle only: N (N +
+// 1) / 2 threads with a 5 x 5 tile each in registers (m <= 100: 210 threads,
+// 100 registers of tile), and inverts it in place by the symmetric sweep.
+// Panel by panel of 5 pivots P, with R = A_P. and G the swept panel (A_PP^-1
+// R, and A_PP^-1 itself in the columns of P):
+//   A_ij -= R_Pi^T G_Pj (i, j off P);  A_Pj = G_Pj;  A_PP = -G_PP,
+// after which A = -S^-1.  A panel's own sweep is a chain of 5 reciprocals, so
+// it runs one panel ahead in warps of its own: the tile threads publish the
+// next panel's entries before they apply panel k, and the panel warps apply
+// panel k to those 5 rows themselves and sweep them meanwhile.  The
+// right-hand side rides along as one more column of the panels.
+//
+// Bound by FP64 arithmetic for long lines (half of m^3 complex multiply-adds
+// a line) and by the panels' chains for short ones.  One polarisation, against
+// the band elimination of k_bc2d (a pivot at a time, two block barriers and
+// the whole window through shared memory for each): 200 x 200 x 100 cells 18.9
+// against 208.4 ms, 101 x 83 x 61 1.8 against 17.8 ms, 40^3 0.43 against
+// 4.66 ms.  The error against dense 64-bit solves is the same (2e-14).
+// ---------------------------------------------------------------------------
+constexpr int kBcT = 5;                  // tile edge and panel width
+constexpr int kBcMaxN = 20;              // tiles along a line
+constexpr int kBcMaxM = kBcT * kBcMaxN;  // longest line
+constexpr int kBcOwn = 32 - kBcT;        // columns of a panel per panel warp; the other lanes hold the pivots'
+constexpr int kBcMaxThreads = 352;
+
+__host__ __device__ constexpr int bc_tiles(int N) { return N * (N + 1) / 2; }
+__host__ __device__ constexpr int bc_tile_warps(int N) { return (bc_tiles(N) + 31) / 32; }
+__host__ __device__ constexpr int bc_panel_warps(int N) { return (kBcT * N + 1 + kBcOwn - 1) / kBcOwn; }
+__host__ __device__ constexpr int bc_sweep_threads(int N) { return 32 * (bc_tile_warps(N) + bc_panel_warps(N)); }
+static_assert(bc_sweep_threads(kBcMaxN) <= kBcMaxThreads, "threads of the longest lines");
+// shared memory in double2: R and G of two panels, the raw panel, f, the
+// diagonal, and (doubles) the coupling within the line and to the two sides
+__host__ __device__ constexpr size_t bc_sweep_smem(int N)
+{
+    return (4 * (size_t)kBcT * (kBcT * N + 1) + (size_t)kBcT * kBcT * N + 2 * (size_t)kBcT * N) * 16 +
+           3 * (size_t)kBcT * N * 8;
+}
+static_assert(bc_sweep_smem(kBcMaxN) <= 48 * 1024, "static shared-memory limit");
+
+namespace {
+// tile t of the lower triangle -> (row, column) of tiles
+__device__ __forceinline__ void bc_tile_of(int t, int &ty, int &tx)
+{
+    ty = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+    while (ty * (ty + 1) / 2 > t) ty--;
+    while ((ty + 1) * (ty + 2) / 2 <= t) ty++;
+    tx = t - ty * (ty + 1) / 2;
+}
+__device__ __forceinline__ double2 shfl2(double2 v, int src)
+{
+    return c2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ void cms(double2 &a, double2 b, double2 c)  // a -= b c
+{
+    a.x = fma(-b.x, c.x, fma(b.y, c.y, a.x));
+    a.y = fma(-b.x, c.y, fma(-b.y, c.x, a.y));
+}
+}  // namespace
+
+// mid: the middle line of every slice, from the lines on its two sides;
+// otherwise block 2 s + side eliminates side `side` of slice s
+template <bool mid> __global__ void __launch_bounds__(kBcMaxThreads) k_bc_sweep(BcArgs a)
+{
+    extern __shared__ double2 sm[];
+    constexpr int T = kBcT;
+    const int N = a.N, MP = T * N, MA = MP + 1, m = a.m, n = a.n, NT = bc_tiles(N);
+    double2 *Rb = sm, *Gb = Rb + 2 * T * MA, *Q = Gb + 2 * T * MA, *f = Q + T * MP, *dg = f + MP;
+    double *cs = reinterpret_cast<double *>(dg + MP), *cs2 = cs + MP, *zc = cs2 + MP;
+    const int sl = mid ? blockIdx.x : blockIdx.x >> 1, side = mid ? 0 : blockIdx.x & 1;
+    const int cm_ = n / 2;  // the middle line
+    const int steps = mid ? 1 : side ? n - 1 - cm_ : cm_;
+    if (steps == 0) return;
+    const size_t base = (size_t)sl * n * m;
+    const double2 *cd = a.cd + base, *cb = a.cb + base;
+    const double *cin = a.czc + base, *cout = a.cyc + base;
+    double2 *inv = a.inv + (size_t)sl * n * T * T * NT, *y = a.y + base;
+    const int tw = bc_tile_warps(N) * 32, tid = threadIdx.x;
+    const bool panel = tid >= tw, live = tid < NT;
+    const int pt = tid - tw, pw = pt >> 5, lane = tid & 31;
+    const bool mine = panel && pt < MP;  // the panel thread of unknown pt
+    int ty = 0, tx = 0;
+    if (live) bc_tile_of(tid, ty, tx);
+    auto line = [&](int st) { return mid ? cm_ : side ? n - 1 - st : st; };
+
+    // coefficients of unknown pt of a line; unknowns past m are an identity
+    struct Col {
+        double2 d, b;
+        double z, c, c2;
+    };
+    auto load = [&](int q, bool prev) {
+        Col v{c2(1, 0), c2(0, 0), 0, 0, 0};
+        if (pt < m) {
+            v.d = cd[(size_t)q * m + pt];
+            v.b = cb[(size_t)q * m + pt];
+            v.z = cin[(size_t)q * m + pt];
+            if (mid || prev) v.c = cout[(size_t)(mid || !side ? q - 1 : q) * m + pt];
+            if (mid && q + 1 < n) v.c2 = cout[(size_t)q * m + pt];
+        }
+        return v;
+    };
+    Col nx{};
+    if (mine) {
+        nx = load(line(0), false);
+        if (mid && pt < m) {
+            const double2 yl = y[(size_t)(cm_ - 1) * m + pt];
+            nx.b = c2(nx.b.x - nx.c * yl.x, nx.b.y - nx.c * yl.y);
+            if (cm_ + 1 < n) {
+                const double2 yr = y[(size_t)(cm_ + 1) * m + pt];
+                nx.b = c2(nx.b.x - nx.c2 * yr.x, nx.b.y - nx.c2 * yr.y);
+            }
+        }
+        f[pt] = nx.b;
+        dg[pt] = nx.d;
+        zc[pt] = nx.z;
+        cs[pt] = nx.c;
+        cs2[pt] = nx.c2;
+    }
+    __syncthreads();
+
+    double2 A[T][T];
+    auto publish = [&](int k) {  // panel k's entries as they stand
+        if (!live) return;
+        if (ty == k) {
+#pragma unroll
+            for (int i = 0; i < T; i++)
+#pragma unroll
+                for (int j = 0; j < T; j++) Q[i * MP + tx * T + j] = A[i][j];
+        } else if (tx == k) {
+#pragma unroll
+            for (int i = 0; i < T; i++)
+#pragma unroll
+                for (int j = 0; j < T; j++) Q[j * MP + ty * T + i] = A[i][j];
+        }
+    };
+    // the tile threads arrive, the panel threads wait: the raw panel is there
+    auto raw_arrive = [&]() { asm volatile("bar.arrive 1, %0;" ::"r"(blockDim.x) : "memory"); };
+    auto raw_wait = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x) : "memory"); };
+    // R and G of panel k from the raw panel, panel k - 1 applied first
+    auto sweep = [&](int k) {
+        const int own = pw * kBcOwn + lane, P = k * T, K = P - T;
+        const bool dup = lane >= kBcOwn, ok = dup || own <= MP;
+        const int col = dup ? P + lane - kBcOwn : own;
+        const double2 *R = Rb + ((k - 1) & 1) * T * MA, *G = Gb + ((k - 1) & 1) * T * MA;
+        double2 *Rn = Rb + (k & 1) * T * MA, *Gn = Gb + (k & 1) * T * MA;
+        double2 v[T];
+#pragma unroll
+        for (int r = 0; r < T; r++) v[r] = !ok ? c2(0, 0) : col == MP ? f[P + r] : Q[r * MP + col];
+        if (k > 0 && ok && col < MP) {
+            if (col >= K && col < P) {
+#pragma unroll
+                for (int r = 0; r < T; r++) v[r] = G[(col - K) * MA + P + r];
+            } else {
+#pragma unroll
+                for (int p = 0; p < T; p++) {
+                    const double2 g = G[p * MA + col];
+#pragma unroll
+                    for (int r = 0; r < T; r++) cms(v[r], R[p * MA + P + r], g);
+                }
+            }
+        }
+        if (!dup && ok)
+#pragma unroll
+            for (int r = 0; r < T; r++) Rn[r * MA + col] = v[r];
+#pragma unroll
+        for (int p = 0; p < T; p++) {
+            double2 l[T];
+#pragma unroll
+            for (int r = 0; r < T; r++) l[r] = shfl2(v[r], kBcOwn + p);
+            // the pivots are of the size of ratios of cell widths and of omega
+            // mu sigma times a cell's area: their squares neither overflow nor vanish
+            const double den = __drcp_rn(fma(l[p].x, l[p].x, l[p].y * l[p].y));
+            const double2 iv = c2(l[p].x * den, -l[p].y * den);
+            const bool pc = col == P + p;
+            const double2 g = pc ? iv : cm(v[p], iv);
+#pragma unroll
+            for (int r = 0; r < T; r++) {
+                if (r == p) continue;
+                if (pc) v[r] = c2(0, 0);
+                cms(v[r], l[r], g);
+            }
+            v[p] = g;
+        }
+        if (!dup && ok)
+#pragma unroll
+            for (int r = 0; r < T; r++) Gn[r * MA + col] = v[r];
+    };
+
+    for (int st = 0; st < steps; st++) {
+        const int q = line(st);
+        if (live) {
+#pragma unroll
+            for (int i = 0; i < T; i++)
+#pragma unroll
+                for (int j = 0; j < T; j++) {
+                    const int r = ty * T + i, c = tx * T + j;
+                    double2 v = c2(0, 0);
+                    if (mid) {
+                        const size_t e = (size_t)(i * T + j) * NT + tid, ln = (size_t)T * T * NT;
+                        const double2 u = inv[(size_t)(q - 1) * ln + e];
+                        const double w = cs[r] * cs[c];
+                        v = c2(w * u.x, w * u.y);
+                        if (q + 1 < n) {
+                            const double2 u2 = inv[(size_t)(q + 1) * ln + e];
+                            const double w2 = cs2[r] * cs2[c];
+                            v = c2(v.x + w2 * u2.x, v.y + w2 * u2.y);
+                        }
+                    } else if (st) {
+                        const double w = cs[r] * cs[c];
+                        v = c2(w * A[i][j].x, w * A[i][j].y);
+                    }
+                    if (r == c) v = c2(v.x + dg[r].x, v.y + dg[r].y);
+                    if (r == c + 1) v.x += zc[c];
+                    if (c == r + 1) v.x += zc[r];
+                    A[i][j] = v;
+                }
+        }
+        const bool more = st + 1 < steps;
+        if (panel) {
+            if (mine && more) nx = load(line(st + 1), true);
+            raw_wait();
+            sweep(0);
+        } else {
+            publish(0);
+            raw_arrive();
+        }
+        __syncthreads();
+        for (int k = 0; k < N; k++) {
+            const double2 *R = Rb + (k & 1) * T * MA, *G = Gb + (k & 1) * T * MA;
+            const int P = k * T;
+            if (panel) {
+                if (mine) {  // the right-hand side
+                    double2 v = f[pt];
+                    if (pt >= P && pt < P + T) v = G[(pt - P) * MA + MP];
+                    else
+#pragma unroll
+                        for (int p = 0; p < T; p++) cms(v, R[p * MA + pt], G[p * MA + MP]);
+                    f[pt] = v;
+                }
+                if (k + 1 < N) {
+                    raw_wait();
+                    sweep(k + 1);
+                }
+            } else {
+                if (k + 1 < N) {
+                    publish(k + 1);
+                    raw_arrive();
+                }
+                if (live) {
+                    if (ty != k && tx != k) {
+#pragma unroll
+                        for (int p = 0; p < T; p++) {
+                            double2 g[T];
+#pragma unroll
+                            for (int j = 0; j < T; j++) g[j] = G[p * MA + tx * T + j];
+#pragma unroll
+                            for (int i = 0; i < T; i++) {
+                                const double2 r = R[p * MA + ty * T + i];
+#pragma unroll
+                                for (int j = 0; j < T; j++) cms(A[i][j], r, g[j]);
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < T; i++)
+#pragma unroll
+                            for (int j = 0; j < T; j++) {
+                                const double2 v = ty == k ? G[i * MA + tx * T + j] : G[j * MA + ty * T + i];
+                                A[i][j] = ty == tx ? c2(-v.x, -v.y) : v;
+                            }
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        // A = -S^-1, f = y
+        if (mine) {
+            const double2 v = f[pt];
+            if (pt < m) y[(size_t)q * m + pt] = v;
+            if (more) {
+                f[pt] = c2(nx.b.x - nx.c * v.x, nx.b.y - nx.c * v.y);
+                dg[pt] = nx.d;
+                zc[pt] = nx.z;
+                cs[pt] = nx.c;
+            }
+        }
+        if (live && !mid) {
+            double2 *o = inv + (size_t)q * T * T * NT + tid;
+#pragma unroll
+            for (int i = 0; i < T; i++)
+#pragma unroll
+                for (int j = 0; j < T; j++) o[(size_t)(i * T + j) * NT] = A[i][j];
+        }
+        __syncthreads();
+    }
+}
+
+// x_q = y_q + A_q (C x_{q -+ 1}) outwards from the middle line, block 2 s +
+// side; A_q = -S_q^-1 in tiles as k_bc_sweep left it, read once.  A tile
+// serves its rows and, by symmetry, its columns; the partial sums of a row
+// are added in the order of the tiles.  Block 2 s also writes the middle line
+// and the boundary nodes of E0: side columns, 1 along the top; the bottom row
+// stays zero.
+__global__ void __launch_bounds__(256) k_bc_subst(BcArgs a)
+{
+    extern __shared__ double2 sm[];
+    constexpr int T = kBcT;
+    const int N = a.N, MP = T * N, MA = MP + 1, m = a.m, n = a.n, NT = bc_tiles(N), tid = threadIdx.x;
+    double2 *v = sm, *part = sm + MP;
+    const int q0 = blockIdx.x >> 1, side = blockIdx.x & 1, s = a.slice0 + q0, cm_ = n / 2;
+    const Slice sl(a, s);
+    const size_t base = (size_t)q0 * n * m;
+    const double2 *y = a.y + base, *inv = a.inv + (size_t)q0 * n * T * T * NT;
+    const double *cout = a.cyc + base;
+    auto edge = [&](int q, int b) { return a.rows ? sl.edge(b + 1, q + 1) : sl.edge(q + 1, b + 1); };
+    if (side == 0) {
+        const double2 *left = a.side + (size_t)s * 2 * (a.nz + 1), *right = left + (a.nz + 1);
+        for (int k = tid; k < a.nz; k += blockDim.x) {
+            a.e0[sl.edge(0, k)] = left[k];
+            a.e0[sl.edge(a.nh, k)] = right[k];
+        }
+        for (int h = 1 + tid; h < a.nh; h += blockDim.x) a.e0[sl.edge(h, 0)] = c2(1.0, 0.0);
+        if (tid < m) a.e0[edge(cm_, tid)] = y[(size_t)cm_ * m + tid];
+    }
+    const int steps = side ? n - 1 - cm_ : cm_;
+    if (steps == 0) return;
+    const bool live = tid < NT, mine = tid < MP;
+    int ty = 0, tx = 0;
+    if (live) bc_tile_of(tid, ty, tx);
+    auto line = [&](int st) { return side ? cm_ + 1 + st : cm_ - 1 - st; };
+    // coupling of line q to its neighbour towards the middle
+    auto coup = [&](int q) { return tid < m ? cout[(size_t)(side ? q - 1 : q) * m + tid] : 0.0; };
+    double2 A[T][T], yq = c2(0, 0);
+    auto load = [&](int q) {
+        if (live) {
+            const double2 *p = inv + (size_t)q * T * T * NT + tid;
+#pragma unroll
+            for (int i = 0; i < T; i++)
+#pragma unroll
+                for (int j = 0; j < T; j++) A[i][j] = p[(size_t)(i * T + j) * NT];
+        }
+        if (mine && tid < m) yq = y[(size_t)q * m + tid];
+    };
+    load(line(0));
+    if (mine) {
+        const double c = coup(line(0));
+        const double2 x = tid < m ? y[(size_t)cm_ * m + tid] : c2(0, 0);
+        v[tid] = c2(c * x.x, c * x.y);
+    }
+    __syncthreads();
+    for (int st = 0; st < steps; st++) {
+        const int q = line(st);
+        const bool more = st + 1 < steps;
+        if (live) {
+            double2 pr[T], pc[T];
+#pragma unroll
+            for (int i = 0; i < T; i++) pr[i] = pc[i] = c2(0, 0);
+#pragma unroll
+            for (int i = 0; i < T; i++) {
+                const double2 vi = v[ty * T + i];
+#pragma unroll
+                for (int j = 0; j < T; j++) {
+                    const double2 w = A[i][j], vj = v[tx * T + j];
+                    pr[i].x += w.x * vj.x - w.y * vj.y;
+                    pr[i].y += w.x * vj.y + w.y * vj.x;
+                    pc[j].x += w.x * vi.x - w.y * vi.y;
+                    pc[j].y += w.x * vi.y + w.y * vi.x;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < T; i++) part[tx * MA + ty * T + i] = pr[i];
+            if (ty != tx)
+#pragma unroll
+                for (int i = 0; i < T; i++) part[ty * MA + tx * T + i] = pc[i];
+        }
+        const double2 yc = yq;
+        if (more) load(line(st + 1));  // ahead of their use
+        const double cn = more && mine ? coup(line(st + 1)) : 0.0;
+        __syncthreads();
+        if (mine) {
+            double2 x = yc;
+            for (int t = 0; t < N; t++) {
+                const double2 p = part[t * MA + tid];
+                x = c2(x.x + p.x, x.y + p.y);
+            }
+            if (tid < m) a.e0[edge(q, tid)] = x;
+            v[tid] = c2(cn * x.x, cn * x.y);
+        }
+        __syncthreads();
+    }
 }
 
 // One block (32 x BY threads) per slice of the launch chunk.
@@ -461,6 +868,20 @@ void launch_bc1d(const BcArgs &a, cudaStream_t s)
     k_bc1d<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(a);
 }
 
+static size_t bc_subst_smem(int N) { return ((size_t)kBcT * N + (size_t)N * (kBcT * N + 1)) * sizeof(double2); }
+
+// the three launches of the block elimination
+void launch_bc_lines(const BcArgs &a, int nslices, cudaStream_t s)
+{
+    g_launch_count.fetch_add(3, std::memory_order_relaxed);
+    const int th = bc_sweep_threads(a.N);
+    const size_t sm = bc_sweep_smem(a.N);
+    k_bc_sweep<false><<<2 * nslices, th, sm, s>>>(a);
+    k_bc_sweep<true><<<nslices, th, sm, s>>>(a);
+    const int tb = std::max(32 * bc_tile_warps(a.N), (kBcT * a.N + 31) / 32 * 32);
+    k_bc_subst<<<2 * nslices, tb, bc_subst_smem(a.N), s>>>(a);
+}
+
 int launch_bc2d(const BcArgs &a, int nblocks, bool window_in_smem, cudaStream_t s)
 {
     const size_t smem = bc_smem_bytes(a.nz, window_in_smem);
@@ -490,11 +911,20 @@ int Solver::compute_bc(int imode, double om, double *e0, bool device)
     const int64_t n = (int64_t)(nh - 1) * m;
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev_);
-    const bool smem = bc_smem_bytes(nz, true) <= (size_t)optin;
-    // per slice: U rows (n x M), reduced right-hand side (n), diagonal (n),
-    // operator right-hand side (n), the two couplings (2n doubles = n double2),
-    // the window when it is not in shared memory (M x M)
-    const size_t per_slice = ((size_t)n * M + 4 * (size_t)n + (smem ? 0 : (size_t)M * M)) * sizeof(double2);
+    // the block elimination where its lines, along the shorter axis, fit in
+    // registers (10 to 11 times the band elimination's speed at 39, 60 and 99
+    // unknowns a line); its work grows with the cube of their length
+    const bool rows = nh < nz;
+    const int lm = rows ? nh - 1 : m, ln = rows ? m : nh - 1;
+    const bool lines = lm <= kBcMaxM;
+    const int N = (lm + kBcT - 1) / kBcT;
+    const bool smem = lines || bc_smem_bytes(nz, true) <= (size_t)optin;
+    // per slice: U rows (n x M) or the tiles of the lines' inverses, reduced
+    // right-hand side (n), diagonal (n), operator right-hand side (n), the two
+    // couplings (2n doubles = n double2), the window when it is neither in
+    // registers nor in shared memory (M x M)
+    const size_t fact = lines ? (size_t)ln * kBcT * kBcT * bc_tiles(N) : (size_t)n * M;
+    const size_t per_slice = (fact + 4 * (size_t)n + (smem ? 0 : (size_t)M * M)) * sizeof(double2);
     const size_t cap = (size_t)8 << 30;
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>(nslice, cap / per_slice));
     const size_t fixed = ((size_t)nslice * 2 * (nz + 1) + (size_t)nslice * 2 * nz + (size_t)nslice * (nh + 1));
@@ -519,7 +949,11 @@ int Solver::compute_bc(int imode, double om, double *e0, bool device)
     a.side = p; p += (size_t)nslice * 2 * (nz + 1);
     a.cpr = p; p += (size_t)nslice * 2 * nz;
     a.bottom = p; p += (size_t)nslice * (nh + 1);
-    a.U = p; p += (size_t)chunk * n * M;
+    a.rows = lines && rows;
+    a.m = lm;
+    a.n = ln;
+    a.N = N;
+    a.U = a.inv = p; p += (size_t)chunk * fact;
     a.y = p; p += (size_t)chunk * n;
     a.cd = p; p += (size_t)chunk * n;
     a.cb = p; p += (size_t)chunk * n;
@@ -534,10 +968,15 @@ int Solver::compute_bc(int imode, double om, double *e0, bool device)
     for (int s0 = 0; s0 < nslice; s0 += chunk) {
         a.slice0 = s0;
         launch_bc_coef(a, std::min(chunk, nslice - s0), stream_);
+        if (lines) {
+            launch_bc_lines(a, std::min(chunk, nslice - s0), stream_);
+            continue;
+        }
         if ((rc = check((cudaError_t)launch_bc2d(a, std::min(chunk, nslice - s0), smem, stream_), "mt3d_compute_bc")))
             return rc;
         launch_bc_back(a, std::min(chunk, nslice - s0), stream_);
     }
+    if ((rc = check(cudaGetLastError(), "mt3d_compute_bc"))) return rc;
     if (!device &&
         (rc = check(cudaMemcpyAsync(e0, a.e0, nE * sizeof(double2), cudaMemcpyDeviceToHost, stream_), "copy E0")))
         return rc;

@@ -199,16 +199,18 @@ MT3D_API int mt3d_mult_aii(mt3d_handle h, int adjt, const double *x, double *y);
  * x and y are interior vectors (nEi complex doubles, 16-byte aligned) in
  * device memory of the handle's device.  The work is only enqueued on the
  * handle's stream (mt3d_set_stream); y is ready when that stream reaches
- * this point.  The scratch (two full edge vectors, the grad-div node
- * potentials and a state record) is one fixed 16 MiB device array per
- * device: grids whose 256 + 16 * (2 nE + nN) bytes exceed it (about 52^3
- * cells) are rejected with MT3D_INVALID_ARGUMENT.  The first mt3d_create on
- * a device looks up the scratch address (cudaGetSymbolAddress), which is
- * what commits the array's 16 MiB, and loads the kernels of this entry, so
- * this entry takes no device memory on any call; create the handle before a
- * memory pool takes the device's free memory.  The scratch is shared by all
- * handles on a device, so calls whose GPU work overlaps in time (different
- * streams, handles or host threads) race; calls on one stream are safe.
+ * this point.  Where y does not overlap x the product takes one kernel and
+ * no scratch; otherwise it goes through a scratch (two full edge vectors, the
+ * grad-div node potentials and a state record), one fixed 16 MiB device array
+ * per device.  Grids whose 256 + 16 * (2 nE + nN) bytes exceed it (about 52^3
+ * cells) are rejected with MT3D_INVALID_ARGUMENT either way.  The first
+ * mt3d_create on a device looks up the scratch address (cudaGetSymbolAddress),
+ * which is what commits the array's 16 MiB, and loads the kernels of this
+ * entry, so this entry takes no device memory on any call; create the handle
+ * before a memory pool takes the device's free memory.  The scratch is shared
+ * by all handles on a device, so calls with overlapping vectors whose GPU work
+ * overlaps in time (different streams, handles or host threads) race; calls
+ * on one stream are safe.
  * With adjt != 0 the product is the conjugate transpose, as mt3d_mult_aii's. */
 MT3D_API int mt3d_mult_aii_device_noalloc(mt3d_handle h, int adjt, const double *x, double *y);
 

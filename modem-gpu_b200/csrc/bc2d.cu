@@ -249,16 +249,16 @@ __global__ void k_bc_coef(BcArgs a, int nslices)
 // R, and A_PP^-1 itself in the columns of P):
 //   A_ij -= R_Pi^T G_Pj (i, j off P);  A_Pj = G_Pj;  A_PP = -G_PP,
 // after which A = -S^-1.  A panel's own sweep is a chain of 5 reciprocals, so
-// it runs one panel ahead in warps of its own: the tile threads publish the
-// next panel's entries before they apply panel k, and the panel warps apply
-// panel k to those 5 rows themselves and sweep them meanwhile.  The
-// right-hand side rides along as one more column of the panels.
+// it runs one panel ahead in warps of its own: while the tile threads apply
+// panel k, the panel warps apply it to the 5 rows of panel k + 1, which the
+// tile threads published one panel before, and sweep them.  The right-hand
+// side rides along as one more column of the panels.
 //
 // Bound by FP64 arithmetic for long lines (half of m^3 complex multiply-adds
 // a line) and by the panels' chains for short ones.  One polarisation, against
 // the band elimination of k_bc2d (a pivot at a time, two block barriers and
-// the whole window through shared memory for each): 200 x 200 x 100 cells 18.9
-// against 208.4 ms, 101 x 83 x 61 1.8 against 17.8 ms, 40^3 0.43 against
+// the whole window through shared memory for each): 200 x 200 x 100 cells 18.3
+// against 208.4 ms, 101 x 83 x 61 1.7 against 17.8 ms, 40^3 0.39 against
 // 4.66 ms.  The error against dense 64-bit solves is the same (2e-14).
 // ---------------------------------------------------------------------------
 constexpr int kBcT = 5;                  // tile edge and panel width
@@ -266,20 +266,22 @@ constexpr int kBcMaxN = 20;              // tiles along a line
 constexpr int kBcMaxM = kBcT * kBcMaxN;  // longest line
 constexpr int kBcOwn = 32 - kBcT;        // columns of a panel per panel warp; the other lanes hold the pivots'
 constexpr int kBcMaxThreads = 352;
+// up to 60 unknowns a line two blocks fit on an SM, whose chains overlap
+constexpr int kBcPairThreads = 192;
 
 __host__ __device__ constexpr int bc_tiles(int N) { return N * (N + 1) / 2; }
 __host__ __device__ constexpr int bc_tile_warps(int N) { return (bc_tiles(N) + 31) / 32; }
 __host__ __device__ constexpr int bc_panel_warps(int N) { return (kBcT * N + 1 + kBcOwn - 1) / kBcOwn; }
 __host__ __device__ constexpr int bc_sweep_threads(int N) { return 32 * (bc_tile_warps(N) + bc_panel_warps(N)); }
 static_assert(bc_sweep_threads(kBcMaxN) <= kBcMaxThreads, "threads of the longest lines");
-// shared memory in double2: R and G of two panels, the raw panel, f, the
-// diagonal, and (doubles) the coupling within the line and to the two sides
+// shared memory in double2: R, G and the published entries of two panels, f
+// twice, the diagonal, and (doubles) the coupling within the line and to the
+// two sides
 __host__ __device__ constexpr size_t bc_sweep_smem(int N)
 {
-    return (4 * (size_t)kBcT * (kBcT * N + 1) + (size_t)kBcT * kBcT * N + 2 * (size_t)kBcT * N) * 16 +
+    return (4 * (size_t)kBcT * (kBcT * N + 1) + 2 * (size_t)kBcT * kBcT * N + 3 * (size_t)kBcT * N) * 16 +
            3 * (size_t)kBcT * N * 8;
 }
-static_assert(bc_sweep_smem(kBcMaxN) <= 48 * 1024, "static shared-memory limit");
 
 namespace {
 // tile t of the lower triangle -> (row, column) of tiles
@@ -294,6 +296,16 @@ __device__ __forceinline__ double2 shfl2(double2 v, int src)
 {
     return c2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
+// 1 / x for normal x: the hardware's approximation y (2^-23 or better, so e =
+// 1 - x y is small) and the first terms of 1 / x = y (1 + e + e^2 + ...), three
+// dependent operations; what is dropped, e^3, lies below the last bit
+__device__ __forceinline__ double rcp_fast(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
 __device__ __forceinline__ void cms(double2 &a, double2 b, double2 c)  // a -= b c
 {
     a.x = fma(-b.x, c.x, fma(b.y, c.y, a.x));
@@ -303,12 +315,12 @@ __device__ __forceinline__ void cms(double2 &a, double2 b, double2 c)  // a -= b
 
 // mid: the middle line of every slice, from the lines on its two sides;
 // otherwise block 2 s + side eliminates side `side` of slice s
-template <bool mid> __global__ void __launch_bounds__(kBcMaxThreads) k_bc_sweep(BcArgs a)
+template <bool mid, int threads, int blocks> __global__ void __launch_bounds__(threads, blocks) k_bc_sweep(BcArgs a)
 {
     extern __shared__ double2 sm[];
     constexpr int T = kBcT;
     const int N = a.N, MP = T * N, MA = MP + 1, m = a.m, n = a.n, NT = bc_tiles(N);
-    double2 *Rb = sm, *Gb = Rb + 2 * T * MA, *Q = Gb + 2 * T * MA, *f = Q + T * MP, *dg = f + MP;
+    double2 *Rb = sm, *Gb = Rb + 2 * T * MA, *Qb = Gb + 2 * T * MA, *f = Qb + 2 * T * MP, *dg = f + 2 * MP;
     double *cs = reinterpret_cast<double *>(dg + MP), *cs2 = cs + MP, *zc = cs2 + MP;
     const int sl = mid ? blockIdx.x : blockIdx.x >> 1, side = mid ? 0 : blockIdx.x & 1;
     const int cm_ = n / 2;  // the middle line
@@ -361,74 +373,115 @@ template <bool mid> __global__ void __launch_bounds__(kBcMaxThreads) k_bc_sweep(
     }
     __syncthreads();
 
-    double2 A[T][T];
-    auto publish = [&](int k) {  // panel k's entries as they stand
-        if (!live) return;
-        if (ty == k) {
-#pragma unroll
-            for (int i = 0; i < T; i++)
-#pragma unroll
-                for (int j = 0; j < T; j++) Q[i * MP + tx * T + j] = A[i][j];
-        } else if (tx == k) {
-#pragma unroll
-            for (int i = 0; i < T; i++)
-#pragma unroll
-                for (int j = 0; j < T; j++) Q[j * MP + ty * T + i] = A[i][j];
-        }
-    };
-    // the tile threads arrive, the panel threads wait: the raw panel is there
-    auto raw_arrive = [&]() { asm volatile("bar.arrive 1, %0;" ::"r"(blockDim.x) : "memory"); };
-    auto raw_wait = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x) : "memory"); };
-    // R and G of panel k from the raw panel, panel k - 1 applied first
-    auto sweep = [&](int k) {
-        const int own = pw * kBcOwn + lane, P = k * T, K = P - T;
-        const bool dup = lane >= kBcOwn, ok = dup || own <= MP;
-        const int col = dup ? P + lane - kBcOwn : own;
-        const double2 *R = Rb + ((k - 1) & 1) * T * MA, *G = Gb + ((k - 1) & 1) * T * MA;
-        double2 *Rn = Rb + (k & 1) * T * MA, *Gn = Gb + (k & 1) * T * MA;
-        double2 v[T];
-#pragma unroll
-        for (int r = 0; r < T; r++) v[r] = !ok ? c2(0, 0) : col == MP ? f[P + r] : Q[r * MP + col];
-        if (k > 0 && ok && col < MP) {
-            if (col >= K && col < P) {
-#pragma unroll
-                for (int r = 0; r < T; r++) v[r] = G[(col - K) * MA + P + r];
-            } else {
-#pragma unroll
-                for (int p = 0; p < T; p++) {
-                    const double2 g = G[p * MA + col];
-#pragma unroll
-                    for (int r = 0; r < T; r++) cms(v[r], R[p * MA + P + r], g);
-                }
-            }
-        }
-        if (!dup && ok)
-#pragma unroll
-            for (int r = 0; r < T; r++) Rn[r * MA + col] = v[r];
-#pragma unroll
-        for (int p = 0; p < T; p++) {
-            double2 l[T];
-#pragma unroll
-            for (int r = 0; r < T; r++) l[r] = shfl2(v[r], kBcOwn + p);
-            // the pivots are of the size of ratios of cell widths and of omega
-            // mu sigma times a cell's area: their squares neither overflow nor vanish
-            const double den = __drcp_rn(fma(l[p].x, l[p].x, l[p].y * l[p].y));
-            const double2 iv = c2(l[p].x * den, -l[p].y * den);
-            const bool pc = col == P + p;
-            const double2 g = pc ? iv : cm(v[p], iv);
-#pragma unroll
-            for (int r = 0; r < T; r++) {
-                if (r == p) continue;
-                if (pc) v[r] = c2(0, 0);
-                cms(v[r], l[r], g);
-            }
-            v[p] = g;
-        }
-        if (!dup && ok)
-#pragma unroll
-            for (int r = 0; r < T; r++) Gn[r * MA + col] = v[r];
+    // the block's barrier, reached by the two roles at places of their own
+    auto all_sync = [&]() {
+        __syncwarp();
+        asm volatile("bar.sync 0;" ::: "memory");
     };
 
+    if (panel) {
+        // R and G of panel k from the published entries, panel k - 1 applied first
+        const int own = pw * kBcOwn + lane;
+        const bool dup = lane >= kBcOwn, ok = dup || own <= MP;
+        auto sweep = [&](int k) {
+            const int P = k * T, K = P - T, col = dup ? P + lane - kBcOwn : own;
+            const double2 *R = Rb + ((k - 1) & 1) * T * MA, *G = Gb + ((k - 1) & 1) * T * MA;
+            double2 *Rn = Rb + (k & 1) * T * MA, *Gn = Gb + (k & 1) * T * MA;
+            const double2 *Q = Qb + (k & 1) * T * MP, *fo = f + (k > 0 ? ((k - 1) & 1) * MP : 0);
+            double2 v[T];
+#pragma unroll
+            for (int r = 0; r < T; r++) v[r] = !ok ? c2(0, 0) : col == MP ? fo[P + r] : Q[r * MP + col];
+            if (k > 0 && ok) {
+                if (col >= K && col < P) {
+#pragma unroll
+                    for (int r = 0; r < T; r++) v[r] = G[(col - K) * MA + P + r];
+                } else {
+#pragma unroll
+                    for (int p = 0; p < T; p++) {
+                        const double2 g = G[p * MA + col];
+#pragma unroll
+                        for (int r = 0; r < T; r++) cms(v[r], R[p * MA + P + r], g);
+                    }
+                }
+            }
+            if (!dup && ok)
+#pragma unroll
+                for (int r = 0; r < T; r++) Rn[r * MA + col] = v[r];
+#pragma unroll
+            for (int p = 0; p < T; p++) {
+                double2 l[T];
+#pragma unroll
+                for (int r = 0; r < T; r++) l[r] = shfl2(v[r], kBcOwn + p);
+                // the pivots are of the size of ratios of cell widths and of omega
+                // mu sigma times a cell's area: their squares neither overflow nor vanish
+                const double den = rcp_fast(fma(l[p].x, l[p].x, l[p].y * l[p].y));
+                const double2 iv = c2(l[p].x * den, -l[p].y * den);
+                const bool pc = col == P + p;
+                const double2 g = pc ? iv : cm(v[p], iv);
+#pragma unroll
+                for (int r = 0; r < T; r++) {
+                    if (r == p) continue;
+                    if (pc) v[r] = c2(0, 0);
+                    cms(v[r], l[r], g);
+                }
+                v[p] = g;
+            }
+            if (!dup && ok)
+#pragma unroll
+                for (int r = 0; r < T; r++) Gn[r * MA + col] = v[r];
+        };
+        for (int st = 0; st < steps; st++) {
+            const bool more = st + 1 < steps;
+            if (mine && more) nx = load(line(st + 1), true);
+            all_sync();  // panels 0 and 1 are published
+            sweep(0);
+            all_sync();
+            for (int k = 0; k < N; k++) {
+                const double2 *R = Rb + (k & 1) * T * MA, *G = Gb + (k & 1) * T * MA;
+                const int P = k * T;
+                if (mine) {  // the right-hand side
+                    double2 v = f[(k & 1) * MP + pt];
+                    if (pt >= P && pt < P + T) v = G[(pt - P) * MA + MP];
+                    else
+#pragma unroll
+                        for (int p = 0; p < T; p++) cms(v, R[p * MA + pt], G[p * MA + MP]);
+                    f[((k + 1) & 1) * MP + pt] = v;
+                }
+                if (k + 1 < N) sweep(k + 1);
+                all_sync();
+            }
+            if (mine) {  // f = y; the next line's coefficients
+                const double2 v = f[(N & 1) * MP + pt];
+                if (pt < m) y[(size_t)line(st) * m + pt] = v;
+                if (more) {
+                    f[pt] = c2(nx.b.x - nx.c * v.x, nx.b.y - nx.c * v.y);
+                    dg[pt] = nx.d;
+                    zc[pt] = nx.z;
+                    cs[pt] = nx.c;
+                }
+            }
+            all_sync();
+        }
+        return;
+    }
+
+    double2 A[T][T];
+    auto publish = [&](int k) {  // panel k's entries as they stand
+        double2 *Q = Qb + (k & 1) * T * MP;
+        if (live && k < N) {
+            if (ty == k) {
+#pragma unroll
+                for (int i = 0; i < T; i++)
+#pragma unroll
+                    for (int j = 0; j < T; j++) Q[i * MP + tx * T + j] = A[i][j];
+            } else if (tx == k) {
+#pragma unroll
+                for (int i = 0; i < T; i++)
+#pragma unroll
+                    for (int j = 0; j < T; j++) Q[j * MP + ty * T + i] = A[i][j];
+            }
+        }
+    };
     for (int st = 0; st < steps; st++) {
         const int q = line(st);
         if (live) {
@@ -458,83 +511,47 @@ template <bool mid> __global__ void __launch_bounds__(kBcMaxThreads) k_bc_sweep(
                     A[i][j] = v;
                 }
         }
-        const bool more = st + 1 < steps;
-        if (panel) {
-            if (mine && more) nx = load(line(st + 1), true);
-            raw_wait();
-            sweep(0);
-        } else {
-            publish(0);
-            raw_arrive();
-        }
-        __syncthreads();
+        publish(0);
+        publish(1);
+        all_sync();
+        all_sync();  // panel 0 is swept
         for (int k = 0; k < N; k++) {
             const double2 *R = Rb + (k & 1) * T * MA, *G = Gb + (k & 1) * T * MA;
-            const int P = k * T;
-            if (panel) {
-                if (mine) {  // the right-hand side
-                    double2 v = f[pt];
-                    if (pt >= P && pt < P + T) v = G[(pt - P) * MA + MP];
-                    else
+            if (live) {
+                if (ty != k && tx != k) {
 #pragma unroll
-                        for (int p = 0; p < T; p++) cms(v, R[p * MA + pt], G[p * MA + MP]);
-                    f[pt] = v;
-                }
-                if (k + 1 < N) {
-                    raw_wait();
-                    sweep(k + 1);
-                }
-            } else {
-                if (k + 1 < N) {
-                    publish(k + 1);
-                    raw_arrive();
-                }
-                if (live) {
-                    if (ty != k && tx != k) {
+                    for (int p = 0; p < T; p++) {
+                        double2 g[T];
 #pragma unroll
-                        for (int p = 0; p < T; p++) {
-                            double2 g[T];
+                        for (int j = 0; j < T; j++) g[j] = G[p * MA + tx * T + j];
 #pragma unroll
-                            for (int j = 0; j < T; j++) g[j] = G[p * MA + tx * T + j];
+                        for (int i = 0; i < T; i++) {
+                            const double2 r = R[p * MA + ty * T + i];
 #pragma unroll
-                            for (int i = 0; i < T; i++) {
-                                const double2 r = R[p * MA + ty * T + i];
-#pragma unroll
-                                for (int j = 0; j < T; j++) cms(A[i][j], r, g[j]);
-                            }
+                            for (int j = 0; j < T; j++) cms(A[i][j], r, g[j]);
                         }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < T; i++)
-#pragma unroll
-                            for (int j = 0; j < T; j++) {
-                                const double2 v = ty == k ? G[i * MA + tx * T + j] : G[j * MA + ty * T + i];
-                                A[i][j] = ty == tx ? c2(-v.x, -v.y) : v;
-                            }
                     }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < T; i++)
+#pragma unroll
+                        for (int j = 0; j < T; j++) {
+                            const double2 v = ty == k ? G[i * MA + tx * T + j] : G[j * MA + ty * T + i];
+                            A[i][j] = ty == tx ? c2(-v.x, -v.y) : v;
+                        }
                 }
             }
-            __syncthreads();
+            publish(k + 2);
+            all_sync();
         }
-        // A = -S^-1, f = y
-        if (mine) {
-            const double2 v = f[pt];
-            if (pt < m) y[(size_t)q * m + pt] = v;
-            if (more) {
-                f[pt] = c2(nx.b.x - nx.c * v.x, nx.b.y - nx.c * v.y);
-                dg[pt] = nx.d;
-                zc[pt] = nx.z;
-                cs[pt] = nx.c;
-            }
-        }
-        if (live && !mid) {
+        if (live && !mid) {  // A = -S^-1
             double2 *o = inv + (size_t)q * T * T * NT + tid;
 #pragma unroll
             for (int i = 0; i < T; i++)
 #pragma unroll
                 for (int j = 0; j < T; j++) o[(size_t)(i * T + j) * NT] = A[i][j];
         }
-        __syncthreads();
+        all_sync();
     }
 }
 
@@ -870,14 +887,24 @@ void launch_bc1d(const BcArgs &a, cudaStream_t s)
 
 static size_t bc_subst_smem(int N) { return ((size_t)kBcT * N + (size_t)N * (kBcT * N + 1)) * sizeof(double2); }
 
+template <int threads, int blocks> static void bc_sweep_launch(const BcArgs &a, int nslices, cudaStream_t s)
+{
+    const int th = bc_sweep_threads(a.N);
+    const size_t sm = bc_sweep_smem(a.N);
+    if (sm > 48 * 1024) {
+        cudaFuncSetAttribute(k_bc_sweep<false, threads, blocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaFuncSetAttribute(k_bc_sweep<true, threads, blocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    }
+    k_bc_sweep<false, threads, blocks><<<2 * nslices, th, sm, s>>>(a);
+    k_bc_sweep<true, threads, blocks><<<nslices, th, sm, s>>>(a);
+}
+
 // the three launches of the block elimination
 void launch_bc_lines(const BcArgs &a, int nslices, cudaStream_t s)
 {
     g_launch_count.fetch_add(3, std::memory_order_relaxed);
-    const int th = bc_sweep_threads(a.N);
-    const size_t sm = bc_sweep_smem(a.N);
-    k_bc_sweep<false><<<2 * nslices, th, sm, s>>>(a);
-    k_bc_sweep<true><<<nslices, th, sm, s>>>(a);
+    if (bc_sweep_threads(a.N) <= kBcPairThreads) bc_sweep_launch<kBcPairThreads, 2>(a, nslices, s);
+    else bc_sweep_launch<kBcMaxThreads, 1>(a, nslices, s);
     const int tb = std::max(32 * bc_tile_warps(a.N), (kBcT * a.N + 31) / 32 * 32);
     k_bc_subst<<<2 * nslices, tb, bc_subst_smem(a.N), s>>>(a);
 }

@@ -676,8 +676,8 @@ template <int stage, bool gd> static void launch_hat_vt_t(const KArgs<float> &a,
 {
     const size_t sm = sizeof(TmaSmem);
     const int res = tma_resident(kh_vt<stage, gd>, sm, 2 + 2 * stage + (gd ? 1 : 0), kHatThreads);
-    kh_vt<stage, gd><<<dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, res)), kHatThreads, sm, s>>>(tp,
-                                                                                                              a);
+    kh_vt<stage, gd><<<dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kHatThreads, sm, s>>>(
+        tp, a);
 }
 template <int stage> static void launch_hat_stage(const KArgs<float> &a, int nrhs, cudaStream_t s)
 {
@@ -856,6 +856,9 @@ int launch_hat_iter_multi(const KArgs<float> *args, const int *nrhs, const int *
     tma_resident(kh_vt_multi<4>, smb, 20, kHatThreads);
     tma_resident(kh_vt_multi<5>, smb, 21, kHatThreads);
     p.eb0[0] = p.sb0[0] = 0;
+    const auto planes_of = [&](int g) { return (double)nrhs[g] * args[g].cmap.tiles * (args[g].g.nz + 1); };
+    double all = 0.0;
+    for (int g = 0; g < ng; g++) all += planes_of(g);
     for (int g = 0; g < ng; g++) {
         p.a[g] = args[g];
         p.nr[g] = nrhs[g];
@@ -867,7 +870,12 @@ int launch_hat_iter_multi(const KArgs<float> *args, const int *nrhs, const int *
             p.tp[g][w].sig = args[g].tma->sig;
             p.tp[g][w].node = args[g].tma->node;
         }
-        p.zch[g] = zch && zch[g] > 0 ? zch[g] : stage_chunks(args[g].g.nz, args[g].cmap.tiles, res);
+        // a grid's share of the resident blocks is its share of the work; more
+        // chunks than planes would only add empty ones, and the reductions'
+        // partial sums have room for one chunk per plane
+        const int share = std::max(1, (int)(res * (planes_of(g) / all)));
+        p.zch[g] = std::min(zch && zch[g] > 0 ? zch[g] : stage_chunks(args[g].g.nz, args[g].cmap.tiles, share, nrhs[g]),
+                            args[g].g.nz + 1);
         p.eb0[g + 1] = p.eb0[g] + nrhs[g] * args[g].nblk;
         p.sb0[g + 1] = p.sb0[g] + nrhs[g] * args[g].cmap.tiles * p.zch[g];
     }

@@ -200,7 +200,7 @@ void launch_bc_back(const BcArgs &a, int nslices, cudaStream_t s);
 void launch_bc_lines(const BcArgs &a, int nslices, cudaStream_t s);
 int launch_bc2d(const BcArgs &a, int nblocks, bool window_in_smem, cudaStream_t s);
 void launch_nodes_to_padded(const Geo<double> &g, const double *src, PadLayout pl, float *dst, cudaStream_t s);
-int stage_chunks(int nz, int tiles, int resident);
+int stage_chunks(int nz, int tiles, int resident, int nrhs);
 template <typename T> void launch_cocg_iter(const ColArgs<T> &a, int nrhs, cudaStream_t s, cudaEvent_t *ev = nullptr);
 
 template <typename T>

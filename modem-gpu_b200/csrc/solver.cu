@@ -429,8 +429,8 @@ int Solver::ensure_workspace(int nrhs, int precision)
     }
     int c;
     const ColMapHost cm = col_map(nx, ny);
-    const int nb = std::max({blocks_for(nE, c), blocks_for(nN, c), cm.tiles * std::max(1, (nz + 1) / 8),
-                             1184});
+    // partial sums: the stencil launches have up to one chunk per node plane
+    const int nb = std::max({blocks_for(nE, c), blocks_for(nN, c), cm.tiles * (nz + 1), 1184});
     err |= w.bst.alloc(nrhs * sizeof(BicgState)) | w.pst.alloc(nrhs * sizeof(PcgState)) |
            w.ost.alloc(nrhs * sizeof(OuterState)) | w.qst.alloc(nrhs * sizeof(QmrState));
     err |= w.parts.alloc((size_t)nrhs * nb * kMaxParts * sizeof(double)) | w.cnt.alloc(3 * nrhs * sizeof(unsigned));

@@ -6,8 +6,7 @@
 //
 // Grid: blockIdx.x = tile of node columns, blockIdx.y = right-hand side,
 // blockIdx.z = chunk of node planes.  The number of chunks is chosen per
-// launch shape so that the blocks fill the resident slots of the GPU in as
-// few, as full waves as possible (stage_chunks).
+// launch shape (stage_chunks).
 #include <algorithm>
 #include <atomic>
 #include <mutex>
@@ -168,28 +167,58 @@ template <typename K> static int stage_setup(K kern, size_t smem, int slot)
     return occ[dev][slot];
 }
 
-// chunks of node planes: the count that minimises (waves of resident blocks)
-// x (planes per chunk + the 3 planes of the prologue), chunks >= 8 planes.
-// Sized for one right-hand side: the blocks of right-hand sides that have
-// converged exit at once, and the last one left must still fill the GPU.
-int stage_chunks(int nz, int tiles, int resident)
+// Time of a launch of c chunks of len planes (the last of them shorter) over
+// `layer` blocks each, in planes of a block that has its SM to itself.  A block
+// costs two planes to start; blocks that share an SM slow each other down by a
+// fifth each (the fused FP32 stencil: 1.55, 1.85, 2.2 and 2.5 us a plane with
+// one to four blocks, which is latency more than throughput, so a small grid
+// is faster in many short chunks than in few long ones).
+static double stage_time(long layer, int c, int len, int last, long resident)
 {
+    const auto shared = [](long blocks) { return 1.0 + 0.2 * ((blocks + 147) / 148 - 1); };
+    const long L = len + 2, l = last + 2, full = layer * (c - 1);
+    if (layer * c <= resident) return L * shared(layer * c);
+    const long r = full % resident, free_ = resident - r;
+    const double t = (double)(full / resident) * L * shared(resident);
+    if (r == 0) return t + (double)((layer + resident - 1) / resident) * l * shared(std::min(layer, resident));
+    // the short chunks go beside the last r of the others, and what is left after them
+    const long room = free_ * std::max<long>(1, L / l);
+    const long tail = layer <= room ? std::max(L, (layer + free_ - 1) / free_ * l)
+                                    : L + (layer - room + resident - 1) / resident * l;
+    return t + tail * shared(std::min(resident, r + layer));
+}
+
+// chunks of node planes of a stencil launch over nrhs right-hand sides on a
+// GPU that holds `resident` blocks.  The blocks of right-hand sides that have
+// converged exit at once, so the choice weighs the launch with all, half and
+// one of them running.  us a launch of the fused FP32 stencil, against the
+// count for one right-hand side in chunks of at least 8 planes: 24^3 cells, 2
+// right-hand sides 11.6 (23.2); 40^3, 2: 16.2 (23.7); 64 x 64 x 48, 2: 24.4
+// (30.6); 100 x 100 x 60, 2: 48.7 (55.9); 200 x 200 x 100, 1: the same 3 chunks.
+int stage_chunks(int nz, int tiles, int resident, int nrhs)
+{
+    struct Last {
+        int nz = -1, tiles, resident, nrhs, c;
+    };
+    thread_local Last memo;
+    if (memo.nz == nz && memo.tiles == tiles && memo.resident == resident && memo.nrhs == nrhs) return memo.c;
     const int planes = nz + 1;
-    const long per = tiles;
     int best = 1;
     double best_t = 1e300;
-    for (int c = 1; c <= std::max(1, planes / 8); c++) {
-        const long waves = (per * c + resident - 1) / resident;
-        const int len = (planes + c - 1) / c;
-        const double t = (double)waves * (len + 3);
+    for (int len = planes; len >= 1; len--) {
+        const int c = (planes + len - 1) / len, last = planes - (c - 1) * len;
+        if ((planes + c - 1) / c != len) continue;  // the same count in more even chunks comes later
+        double t = 0.0;
+        for (int n : {nrhs, (nrhs + 1) / 2, 1}) t += stage_time((long)n * tiles, c, len, last, resident);
         if (t < best_t - 1e-9) { best_t = t; best = c; }
     }
+    memo = Last{nz, tiles, resident, nrhs, best};
     return best;
 }
 
 template <typename T> static dim3 stage_grid(const KArgs<T> &a, int nrhs, int resident)
 {
-    return dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, resident));
+    return dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, resident, nrhs));
 }
 
 template <typename T> void launch_stage_init(const KArgs<T> &a, int nrhs, cudaStream_t s)

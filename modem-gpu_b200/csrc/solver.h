@@ -197,6 +197,7 @@ class Solver {
     DevBuf sigs64_, sigs32_, gdw64_, gdw32_, gde_, gdn64_, gdn32_;  // grad-div (SP2) data
     DevBuf setup_;  // model parameter, V_C, V_C sigma_C and sigma_C of the operator set-up
     DevBuf bcs_, bce_;  // 2-D boundary-condition scratch and host-bound output
+    DevBuf site_;       // coordinates, sites and functionals of the data functional
     // padded FP32 layout of the TMA-staged kernels: sigma of both
     // formulations, signed node weights, the tensor maps and a device flag
     // that bounded waits set

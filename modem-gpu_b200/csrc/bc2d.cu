@@ -60,6 +60,17 @@ __device__ __forceinline__ double2 cdv(double2 a, double2 b)
     return c2((a.x * r + a.y) / den, (a.y * r - a.x) / den);
 }
 
+// 1 / x for normal x: the hardware's approximation y (2^-23 or better, so e =
+// 1 - x y is small) and the first terms of 1 / x = y (1 + e + e^2 + ...), three
+// dependent operations; what is dropped, e^3, lies below the last bit
+__device__ __forceinline__ double rcp_fast(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
 struct Slice {
     const BcArgs &a;
     int s;
@@ -106,37 +117,64 @@ __global__ void k_bc1d(BcArgs a)
     double2 *cp = side >= 0 ? a.cpr + ((size_t)s * 2 + side) * nz : nullptr;
     double2 *xs = side >= 0 ? a.side + ((size_t)s * 2 + side) * (nz + 1) : nullptr;
     // row j: ad_{j-1} x_{j-1} + ac_j x_j + ad_j x_{j+1} = r_j, r_0 = -au_0
+    // the conductivities and widths of kAhead rows are read ahead of the chain,
+    // whose step is one complex reciprocal (the entries are of the size of
+    // inverse layer thicknesses and of omega mu sigma times a thickness: their
+    // squares neither overflow nor vanish): 40 us for the columns of 40^3
+    // cells, 107 us for 200 x 200 x 100, against 56 and 172 us with the loads
+    // and six divisions a row on the chain
+    constexpr int kAhead = 8;
     double2 cprev = c2(0, 0), dprev = c2(0, 0);
-    double adprev = 0.0, sk = s1(0), dk = dz1(0);
-    for (int j = 0; j < nz; j++) {
-        const double sk1 = s1(j + 1), dk1 = dz1(j + 1);
-        const double au = 2.0 / dk, ad = 2.0 / dk1;
-        const double ss = sk1 * dk1 + sk * dk;
-        const double2 ac = c2(-au - ad, a.omue * ss);
-        const double2 den = c2(ac.x - adprev * cprev.x, ac.y - adprev * cprev.y);
-        const double2 r = j == 0 ? c2(-au, 0.0) : c2(0.0, 0.0);
-        const double2 cj = cdv(c2(ad, 0.0), den);
-        const double2 dj = cdv(c2(r.x - adprev * dprev.x, r.y - adprev * dprev.y), den);
-        if (side >= 0) {
-            cp[j] = cj;
-            xs[j + 1] = dj;
+    double adprev = 0.0, sk = s1(0), dk = dz1(0), au = 2.0 / dk;
+    for (int j0 = 0; j0 < nz; j0 += kAhead) {
+        double sn[kAhead], dn[kAhead], an[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) {
+            sn[q] = s1(min(j0 + q + 1, nz));
+            dn[q] = dz1(min(j0 + q + 1, nz));
         }
-        cprev = cj;
-        dprev = dj;
-        adprev = ad;
-        sk = sk1;
-        dk = dk1;
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) an[q] = 2.0 / dn[q];
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) {
+            const int j = j0 + q;
+            if (j >= nz) break;
+            const double ad = an[q], ss = sn[q] * dn[q] + sk * dk;
+            const double2 den = c2(-au - ad - adprev * cprev.x, a.omue * ss - adprev * cprev.y);
+            const double iv = rcp_fast(fma(den.x, den.x, den.y * den.y));
+            const double2 id = c2(den.x * iv, -den.y * iv);
+            const double2 r = c2((j == 0 ? -au : 0.0) - adprev * dprev.x, -adprev * dprev.y);
+            cprev = c2(ad * id.x, ad * id.y);
+            dprev = cm(r, id);
+            if (side >= 0) {
+                cp[j] = cprev;
+                xs[j + 1] = dprev;
+            }
+            adprev = au = ad;
+            sk = sn[q];
+            dk = dn[q];
+        }
     }
     if (side < 0) {
         a.bottom[(size_t)s * (a.nh + 1) + col] = dprev;  // x at the bottom node = last d'
         return;
     }
     xs[0] = c2(1.0, 0.0);
-    double2 xn = xs[nz];
-    for (int j = nz - 2; j >= 0; j--) {
-        const double2 d = xs[j + 1];
-        xn = c2(d.x - (cp[j].x * xn.x - cp[j].y * xn.y), d.y - (cp[j].x * xn.y + cp[j].y * xn.x));
-        xs[j + 1] = xn;
+    double2 xn = dprev;
+    for (int j0 = nz - 2; j0 >= 0; j0 -= kAhead) {
+        double2 d[kAhead], c[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) {
+            const int j = max(j0 - q, 0);
+            d[q] = xs[j + 1];
+            c[q] = cp[j];
+        }
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) {
+            if (j0 - q < 0) break;
+            xn = c2(d[q].x - (c[q].x * xn.x - c[q].y * xn.y), d[q].y - (c[q].x * xn.y + c[q].y * xn.x));
+            xs[j0 - q + 1] = xn;
+        }
     }
 }
 
@@ -257,9 +295,10 @@ __global__ void k_bc_coef(BcArgs a, int nslices)
 // Bound by FP64 arithmetic for long lines (half of m^3 complex multiply-adds
 // a line) and by the panels' chains for short ones.  One polarisation, against
 // the band elimination of k_bc2d (a pivot at a time, two block barriers and
-// the whole window through shared memory for each): 200 x 200 x 100 cells 18.3
-// against 208.4 ms, 101 x 83 x 61 1.7 against 17.8 ms, 40^3 0.39 against
-// 4.66 ms.  The error against dense 64-bit solves is the same (2e-14).
+// the whole window through shared memory for each): 200 x 200 x 100 cells 18.2
+// against 208.4 ms, 101 x 83 x 61 1.68 against 17.8 ms, 40^3 0.37 against
+// 4.66 ms.  (8 x 8 blocks in FP64 matrix instructions, which run at the same
+// rate, were slower: 20.6 to 27.9 ms for the first.)  The error against dense 64-bit solves is the same (2e-14).
 // ---------------------------------------------------------------------------
 constexpr int kBcT = 5;                  // tile edge and panel width
 constexpr int kBcMaxN = 20;              // tiles along a line
@@ -295,16 +334,6 @@ __device__ __forceinline__ void bc_tile_of(int t, int &ty, int &tx)
 __device__ __forceinline__ double2 shfl2(double2 v, int src)
 {
     return c2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-// 1 / x for normal x: the hardware's approximation y (2^-23 or better, so e =
-// 1 - x y is small) and the first terms of 1 / x = y (1 + e + e^2 + ...), three
-// dependent operations; what is dropped, e^3, lies below the last bit
-__device__ __forceinline__ double rcp_fast(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
 }
 __device__ __forceinline__ void cms(double2 &a, double2 b, double2 c)  // a -= b c
 {
@@ -882,7 +911,8 @@ void launch_bc1d(const BcArgs &a, cudaStream_t s)
 {
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
     const long long nt = (long long)a.nslice * (a.nh + 1);
-    k_bc1d<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(a);
+    // (one warp a block: a small grid's columns spread over more SMs)
+    k_bc1d<<<(unsigned)((nt + 31) / 32), 32, 0, s>>>(a);
 }
 
 static size_t bc_subst_smem(int N) { return ((size_t)kBcT * N + (size_t)N * (kBcT * N + 1)) * sizeof(double2); }

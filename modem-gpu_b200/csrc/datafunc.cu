@@ -11,8 +11,7 @@
 // weights go up in one copy, and the scratch stays with the handle.  (Built
 // on the host with a linear search per coordinate, a sort of the entries by
 // edge and ten allocations, the adjoint sources of 400 sites on 100 x 100 x 60
-// cells took 1.97 ms; here 0.19 ms, some 20 us of it for clearing the two
-// source vectors.)  Site azimuths are zero (the reference's
+// cells took 1.97 ms; here 0.19 ms.)  Site azimuths are zero (the reference's
 // rotate_Model2Data with zero angles).
 #include <algorithm>
 #include <cmath>

@@ -144,18 +144,22 @@ void launch_hat_apply(const KArgs<float> &a, int nrhs, cudaStream_t s);
 // with the polynomial preconditioner: the cycle's iterate x = M^-1 yhat in x0
 // (after launch_bicg_finish); nothing otherwise
 void launch_hat_conv(const KArgs<float> &a, int nrhs, cudaStream_t s);
-// One FP32 cycle of the fused iteration (maxit iterations of launch_hat_iter,
-// or of launch_hat_iter_multi over ng grids) captured as a CUDA graph and
-// replayed while the launch arguments stay the same; the graph is captured
-// on a private stream and launched on the caller's.
+// One FP32 cycle of the fused iteration (up to maxit iterations of
+// launch_hat_iter, or of launch_hat_iter_multi over ng grids, while any
+// right-hand side is running) captured as a CUDA graph and replayed while the
+// launch arguments stay the same; the graph is captured on a private stream
+// and launched on the caller's.  How often its body ran is at hat_loop_count
+// of the first grid.
 struct HatGraph {
     cudaGraphExec_t exec = nullptr;
     cudaStream_t cap = nullptr;
     std::vector<unsigned char> key;
-    long long launches = 0;  // kernel launches in one replay
+    long long launches = 0;  // kernel launches in one run of the loop's body
     void reset();
     ~HatGraph();
 };
+// beside the error word of the bounded waits
+inline int *hat_loop_count(const KArgs<float> &a) { return a.err + 1; }
 // ng = 0: one grid (args[0], nrhs[0]); returns a CUDA error code
 cudaError_t hat_graph_run(HatGraph &hg, const KArgs<float> *args, const int *nrhs, const int *zch, int ng, int maxit,
                           cudaStream_t s);

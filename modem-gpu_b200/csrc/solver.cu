@@ -16,6 +16,7 @@
 namespace mt3d {
 
 std::atomic<long long> g_alloc_count{0};
+extern std::atomic<long long> g_launch_count;
 
 int DevBuf::alloc(size_t bytes)
 {
@@ -195,8 +196,9 @@ int Solver::create(int dev, int nx_, int ny_, int nz_, int nzAir_, const double 
     pl_.Px = (nx + 1 + 3) / 4 * 4;
     pl_.Py = ny + 1;
     pl_.Pz = nz + 1;
-    if (errf_.alloc(sizeof(int))) return fail(8, "mt3d_create: out of device memory");
-    cudaMemset(errf_.as<void>(), 0, sizeof(int));
+    // the error word of the bounded waits and the loop count of the FP32 cycles
+    if (errf_.alloc(2 * sizeof(int))) return fail(8, "mt3d_create: out of device memory");
+    cudaMemset(errf_.as<void>(), 0, 2 * sizeof(int));
     dx_.assign(dx, dx + nx); dy_.assign(dy, dy + ny); dz_.assign(dz, dz + nz);
     deltas(dx_, delX_); deltas(dy_, delY_); deltas(dz_, delZ_);
     // tables: dx dy dz delX delY delZ rdx rdy rdz
@@ -331,9 +333,11 @@ int Solver::tma_ready()
 // a bounded device-side wait gave up (MT3D_DEVICE_TIMEOUT)
 int Solver::check_device_error(const char *what)
 {
-    int e = 0;
-    cudaMemcpy(&e, errf_.as<void>(), sizeof(int), cudaMemcpyDeviceToHost);
-    if (!e) return 0;
+    int e2[2] = {0, 0};
+    cudaMemcpy(e2, errf_.as<void>(), sizeof e2, cudaMemcpyDeviceToHost);
+    if (ran_) g_launch_count.fetch_add(ran_->launches * e2[1], std::memory_order_relaxed);
+    ran_ = nullptr;
+    if (!e2[0]) return 0;
     cudaMemset(errf_.as<void>(), 0, sizeof(int));
     // the blocks that gave up skipped their reductions: clear the counters
     // of the last-block detection for the next call
@@ -689,6 +693,7 @@ int Solver::run_hat(int nrhs, int maxit)
         for (int it = 0; it < maxit; it++) launch_hat_iter(a, nrhs, stream_, next_events(4));
     } else {
         // the cycle as one CUDA graph, replayed while its arguments hold
+        ran_ = &hat_graph_;
         const cudaError_t e = hat_graph_run(hat_graph_, &a, &nrhs, nullptr, 0, maxit, stream_);
         if (e != cudaSuccess) return check(e, "fused BiCGStab graph");
     }
@@ -704,6 +709,7 @@ int Solver::run_hat_multi(const KArgs<float> *args, const int *nrhs, const int *
             if (launch_hat_iter_multi(args, nrhs, zch, ng, s, fp32_events(4))) return 5;
         return 0;
     }
+    ran_ = &hat_graph_multi_;
     return hat_graph_run(hat_graph_multi_, args, nrhs, zch, ng, maxit, s) == cudaSuccess ? 0 : 4;
 }
 

@@ -189,6 +189,7 @@ class Solver {
     std::vector<int> ev_prec_;  // precision of each recorded event
     DevBuf prof_cnt_;           // device sweep counters [FP64, FP32]
     HatGraph hat_graph_, hat_graph_multi_;  // captured FP32 cycles (single grid, multi-grid batch)
+    const HatGraph *ran_ = nullptr;         // the one whose launches are still to be counted
     cudaEvent_t *next_events(int n);
     void collect_events();
     Geo<double> g64_{};

@@ -50,6 +50,10 @@
 
 namespace mt3d {
 
+constexpr int kTX = HatTile::TX, kTY = HatTile::TY, kFW = HatTile::FW, kFR = HatTile::FR, kSW = HatTile::SW,
+              kNW = HatTile::NW, kPhX = HatTile::PhX;
+constexpr unsigned kFBytes = HatTile::FBytes, kSBytes = HatTile::SBytes, kNBytes = HatTile::NBytes;
+
 extern std::atomic<long long> g_launch_count;
 static inline void counted(int n) { g_launch_count.fetch_add(n, std::memory_order_relaxed); }
 
@@ -267,14 +271,14 @@ __device__ __forceinline__ void hat_xr(const KArgs<float> &a, int r, int bx)
 // node of the thread's two columns, padding slots included: yhat =
 // D^-1 (A x)_e and W = |D_e|^2 at interior edges (zero otherwise), e the
 // padded index, aux_e the entry of the vector aux (read one plane ahead,
-// zero when aux is null).  A block of kHatThreads threads covers the 32 x 8
+// zero when aux is null).  A block of kHatThreads threads covers the 16 x 16
 // node tile: thread (tx, ty) takes the node columns (i0 + tx, j0 + ty) and
-// (i0 + tx, j0 + ty + 4), so the per-plane work of a thread (waits,
+// (i0 + tx, j0 + ty + 8), so the per-plane work of a thread (waits,
 // barriers, plane geometry, loop control) is shared by six edges and the
 // register budget of four blocks per SM is 128 per thread.  Returns false
 // (all threads of the block alike) when a wait gave up.
 template <bool gd, typename F>
-__device__ __forceinline__ bool hat_march(TmaSmem &sm, const TmaParams &tp, const Geo<float> &g, PadLayout pl, int r,
+__device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp, const Geo<float> &g, PadLayout pl, int r,
                                           const float2 *__restrict__ aux, float wmu, int i0, int j0, int k0, int k1,
                                           int *err, int limit, F &&f)
 {
@@ -284,7 +288,7 @@ __device__ __forceinline__ bool hat_march(TmaSmem &sm, const TmaParams &tp, cons
     const ColGeo<float> cgA = col_geo(g, min(i, g.nx), min(jA, g.ny));
     const ColGeo<float> cgB = col_geo(g, min(i, g.nx), min(jB, g.ny));
     const int hfA = (ty + 1) * kFW + tx + 2;  // own column in a field plane of the tile
-    const int hsA = (ty + 1) * kSW + tx + 4;  // own column in a sigma plane
+    const int hsA = (ty + 1) * kSW + tx + 1;  // own column in a sigma plane
     const int hnA = ty * kPhX + tx;           // own node in a potential plane
     const int hwA = ty * kNW + tx;            // own node in a node-weight plane
     constexpr int dF = kHatRows * kFW, dS = kHatRows * kSW, dN = kHatRows * kPhX, dW = kHatRows * kNW;
@@ -324,7 +328,7 @@ __device__ __forceinline__ bool hat_march(TmaSmem &sm, const TmaParams &tp, cons
         const unsigned mb = smem_addr(&sm.mbar[s]);
         mbar_expect(mb, tx_bytes + (node ? kNBytes : 0u));
         tma_load4(smem_addr(sm.fld[s]), &tp.in, 2 * (i0 - 2), j0 - 1, p, 3 * r, mb);
-        tma_load4(smem_addr(sm.sig[mod3(p)]), &tp.sig, i0 - 4, j0 - 1, p, 0, mb);
+        tma_load4(smem_addr(sm.sig[mod3(p)]), &tp.sig, i0, j0 - 1, p, 0, mb);
         if (node) tma_load3(smem_addr(sm.nod[p & 1]), &tp.node, i0, j0, p, mb);
     };
     auto wait = [&](int p) -> bool {
@@ -344,9 +348,9 @@ __device__ __forceinline__ bool hat_march(TmaSmem &sm, const TmaParams &tp, cons
     auto phi_plane = [&](int p) {
         const float dZ = (p >= 0 && p <= g.nz) ? g.delZ[p] : 0.f;
         float2 *P = sm.phi[p & 1];
-        P[hnA] = tma_phi_node(sm, g, i, jA, p, tx, ty, cgA.delXi, cgA.delYj, dZ);
-        P[hnA + dN] = tma_phi_node(sm, g, i, jB, p, tx, ty + kHatRows, cgB.delXi, cgB.delYj, dZ);
-        if (hasH) P[hnj * kPhX + hni] = tma_phi_node(sm, g, hi, hj, p, hni, hnj, hdX, hdY, dZ);
+        P[hnA] = tma_phi_node<HatTile>(sm, g, i, jA, p, tx, ty, cgA.delXi, cgA.delYj, dZ);
+        P[hnA + dN] = tma_phi_node<HatTile>(sm, g, i, jB, p, tx, ty + kHatRows, cgB.delXi, cgB.delYj, dZ);
+        if (hasH) P[hnj * kPhX + hni] = tma_phi_node<HatTile>(sm, g, hi, hj, p, hni, hnj, hdX, hdY, dZ);
     };
     const float2 zero = make_float2(0.f, 0.f);
     // signed node weights of each column's nodes (i, j), (i+1, j), (i, j+1)
@@ -542,7 +546,7 @@ __device__ __forceinline__ void hat_vt(const TmaParams &tp, const KArgs<float> &
     if ((!conv && st.status != KS_RUNNING) || !a.ost[r].active) return;
     if (!conv && a.sweeps && threadIdx.x == 0 && bx == 0 && bz == 0) atomicAdd(a.sweeps, 1ULL);
     int i0, j0, k0, k1;
-    tma_tile_at(a.cmap, bx, i0, j0);
+    tma_tile_at<HatTile>(a.hmap, bx, i0, j0);
     tma_range_at(a.g.nz, bz, gz, k0, k1);
     const size_t off = (size_t)r * a.stride;
     float2 *out = (stage == 0 || stage == 3 ? a.v : stage == 2 || stage == 6 ? a.p : stage == 4 ? a.s : a.t) + off;
@@ -558,7 +562,7 @@ __device__ __forceinline__ void hat_vt(const TmaParams &tp, const KArgs<float> &
     // changed the Krylov rounding enough to send more right-hand sides to
     // the FP64 fallback)
     double u[4] = {0.0, 0.0, 0.0, 0.0};
-    TmaSmem &sm = tma_smem();
+    HatTile::Smem &sm = tma_smem<HatTile>();
     const bool ok = hat_march<gd>(
         sm, tp, a.g, a.pl, r, aux, (float)(a.dsgn * a.ost[r].omega * kMu0), i0, j0, k0, k1, a.err, a.wait_limit,
         // y and W are zero at edges that are not interior, and so are x
@@ -584,7 +588,7 @@ __device__ __forceinline__ void hat_vt(const TmaParams &tp, const KArgs<float> &
     if (!ok || !dots) return;
     // the march has read its last staged plane: the field ring is free
     double tot[4];
-    if (block_reduce_last_in<4, kHatThreads>(u, a.parts, a.cnt, r, bx + a.cmap.tiles * bz, a.cmap.tiles * gz, tot,
+    if (block_reduce_last_in<4, kHatThreads>(u, a.parts, a.cnt, r, bx + a.hmap.tiles * bz, a.hmap.tiles * gz, tot,
                                 reinterpret_cast<double *>(sm.fld[0]), reinterpret_cast<int *>(sm.fld[1])) &&
         threadIdx.x == 0) {
         if (kv) {
@@ -651,10 +655,10 @@ template <int stage> __global__ void __launch_bounds__(kHatThreads, 4) kh_vt_mul
 {
     const int g = multi_grid_of(p.sb0, p.ng, blockIdx.x);
     const KArgs<float> &a = p.a[g];
-    const int per = a.cmap.tiles * p.zch[g];
+    const int per = a.hmap.tiles * p.zch[g];
     const int local = blockIdx.x - p.sb0[g];
     const int r = local / per, rem = local - r * per;
-    const int bz = rem / a.cmap.tiles, bx = rem - bz * a.cmap.tiles;
+    const int bz = rem / a.hmap.tiles, bx = rem - bz * a.hmap.tiles;
     const TmaParams &tp = p.tp[g][stage_input(stage)];
     if (a.gd) hat_vt<stage, true>(tp, a, r, bx, bz, p.zch[g]);
     else hat_vt<stage, false>(tp, a, r, bx, bz, p.zch[g]);
@@ -663,6 +667,14 @@ template <int stage> __global__ void __launch_bounds__(kHatThreads, 4) kh_vt_mul
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+ColMapHost hat_map(int nx, int ny)
+{
+    ColMapHost m;
+    m.tiles_x = (nx + 1 + kTX - 1) / kTX;
+    m.tiles = m.tiles_x * ((ny + 1 + kTY - 1) / kTY);
+    return m;
+}
+
 static int hat_grid(long n) { return (int)std::min<long>((n + kThreads - 1) / kThreads, 148L * 16); }
 
 void launch_hat_cast(const KArgs<float> &a, const double2 *r64, size_t stride64, int nrhs, cudaStream_t s)
@@ -674,9 +686,9 @@ void launch_hat_cast(const KArgs<float> &a, const double2 *r64, size_t stride64,
 template <int stage, bool gd> static void launch_hat_vt_t(const KArgs<float> &a, const TmaParams &tp, int nrhs,
                                                            cudaStream_t s)
 {
-    const size_t sm = sizeof(TmaSmem);
+    const size_t sm = sizeof(HatTile::Smem);
     const int res = tma_resident(kh_vt<stage, gd>, sm, 2 + 2 * stage + (gd ? 1 : 0), kHatThreads);
-    kh_vt<stage, gd><<<dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kHatThreads, sm, s>>>(
+    kh_vt<stage, gd><<<dim3(a.hmap.tiles, nrhs, stage_chunks(a.g.nz, a.hmap.tiles, res, nrhs)), kHatThreads, sm, s>>>(
         tp, a);
 }
 template <int stage> static void launch_hat_stage(const KArgs<float> &a, int nrhs, cudaStream_t s)
@@ -685,9 +697,9 @@ template <int stage> static void launch_hat_stage(const KArgs<float> &a, int nrh
     const TmaMaps *m = a.tma;
     TmaParams tp;
     constexpr int in = stage_input(stage);
-    tp.in = in == 0 ? m->ph : in == 1 ? m->sh : in == 2 ? m->pw : in == 3 ? m->sw : m->x0;
-    tp.sig = m->sig;
-    tp.node = m->node;
+    tp.in = in == 0 ? m->hph : in == 1 ? m->hsh : in == 2 ? m->hpw : in == 3 ? m->hsw : m->hx0;
+    tp.sig = m->hsig;
+    tp.node = m->hnode;
     if (a.gd) launch_hat_vt_t<stage, true>(a, tp, nrhs, s);
     else launch_hat_vt_t<stage, false>(a, tp, nrhs, s);
 }
@@ -751,7 +763,7 @@ void launch_hat_conv(const KArgs<float> &a, int nrhs, cudaStream_t s)
 // before a capture (tma_resident calls the runtime only the first time)
 template <int stage> static void hat_prime_stage()
 {
-    const size_t sm = sizeof(TmaSmem);
+    const size_t sm = sizeof(HatTile::Smem);
     tma_resident(kh_vt<stage, false>, sm, 2 + 2 * stage, kHatThreads);
     tma_resident(kh_vt<stage, true>, sm, 3 + 2 * stage, kHatThreads);
     if (stage < 6) tma_resident(kh_vt_multi<(stage < 6 ? stage : 0)>, sm, 16 + stage, kHatThreads);
@@ -908,7 +920,7 @@ int launch_hat_iter_multi(const KArgs<float> *args, const int *nrhs, const int *
     HatMulti p;
     std::memset(&p, 0, sizeof p);
     p.ng = ng;
-    const size_t smb = sizeof(TmaSmem);
+    const size_t smb = sizeof(HatTile::Smem);
     const int res = tma_resident(kh_vt_multi<0>, smb, 16, kHatThreads);
     tma_resident(kh_vt_multi<1>, smb, 17, kHatThreads);
     tma_resident(kh_vt_multi<2>, smb, 18, kHatThreads);
@@ -916,34 +928,34 @@ int launch_hat_iter_multi(const KArgs<float> *args, const int *nrhs, const int *
     tma_resident(kh_vt_multi<4>, smb, 20, kHatThreads);
     tma_resident(kh_vt_multi<5>, smb, 21, kHatThreads);
     p.eb0[0] = p.sb0[0] = 0;
-    const auto planes_of = [&](int g) { return (double)nrhs[g] * args[g].cmap.tiles * (args[g].g.nz + 1); };
+    const auto planes_of = [&](int g) { return (double)nrhs[g] * args[g].hmap.tiles * (args[g].g.nz + 1); };
     double all = 0.0;
     for (int g = 0; g < ng; g++) all += planes_of(g);
     for (int g = 0; g < ng; g++) {
         p.a[g] = args[g];
         p.nr[g] = nrhs[g];
-        p.tp[g][0].in = args[g].tma->ph;
-        p.tp[g][1].in = args[g].tma->sh;
-        p.tp[g][2].in = args[g].tma->pw;
-        p.tp[g][3].in = args[g].tma->sw;
+        p.tp[g][0].in = args[g].tma->hph;
+        p.tp[g][1].in = args[g].tma->hsh;
+        p.tp[g][2].in = args[g].tma->hpw;
+        p.tp[g][3].in = args[g].tma->hsw;
         for (int w = 0; w < 4; w++) {
-            p.tp[g][w].sig = args[g].tma->sig;
-            p.tp[g][w].node = args[g].tma->node;
+            p.tp[g][w].sig = args[g].tma->hsig;
+            p.tp[g][w].node = args[g].tma->hnode;
         }
         // a grid's share of the resident blocks is its share of the work; more
         // chunks than planes would only add empty ones, and the reductions'
         // partial sums have room for one chunk per plane
         const int share = std::max(1, (int)(res * (planes_of(g) / all)));
-        p.zch[g] = std::min(zch && zch[g] > 0 ? zch[g] : stage_chunks(args[g].g.nz, args[g].cmap.tiles, share, nrhs[g]),
+        p.zch[g] = std::min(zch && zch[g] > 0 ? zch[g] : stage_chunks(args[g].g.nz, args[g].hmap.tiles, share, nrhs[g]),
                             args[g].g.nz + 1);
         p.eb0[g + 1] = p.eb0[g] + nrhs[g] * args[g].nblk;
-        p.sb0[g + 1] = p.sb0[g] + nrhs[g] * args[g].cmap.tiles * p.zch[g];
+        p.sb0[g + 1] = p.sb0[g] + nrhs[g] * args[g].hmap.tiles * p.zch[g];
     }
     // the polynomial preconditioner is used when the first grid's handle
     // has it (every handle of a batch shares the control)
     const bool poly = args[0].pc > 0.f;
     counted(poly ? 7 : 5);
-    const size_t sm = sizeof(TmaSmem);
+    const size_t sm = sizeof(HatTile::Smem);
     kh_elem_multi<0><<<p.eb0[ng], kThreads, 0, s>>>(p);
     if (ev) cudaEventRecord(ev[0], s);
     if (poly) {

@@ -18,12 +18,18 @@ struct PadLayout {
     __host__ __device__ long long len() const { return 3LL * Px * Py * Pz; }
 };
 
+// sigma's layout for the tensor copies: as the vectors', one column wider where
+// it has to be, since sigma of column i lies at entry i + 1 (a tile's copy then
+// starts on its 16-byte boundary with the column before the tile)
+inline PadLayout sig_layout(PadLayout pl, int nx) { return PadLayout{(nx + 2 + 3) / 4 * 4, pl.Py, pl.Pz}; }
+
 // tiles of kColX x kColY (i, j) columns for the column-marching kernels
 struct ColMap {
     int tiles_x, tiles;
 };
 using ColMapHost = ColMap;
 ColMapHost col_map(int nx, int ny);
+ColMapHost hat_map(int nx, int ny);  // tiles of the fused FP32 stencil
 
 // arguments of the edge-vector Krylov kernels (one precision T)
 template <typename T> struct KArgs {
@@ -54,7 +60,7 @@ template <typename T> struct KArgs {
     // (grad-div potentials formed inside), 3 TMA-staged on the padded layout;
     // the precomputed inverse diagonal
     int colstencil;
-    ColMap cmap;
+    ColMap cmap, hmap;  // tiles; hmap: of the fused FP32 stencil
     C2<T> *jinv;
     double dsgn;  // ISIGN (-1) for A, +1 for the conjugate transpose
     // entries per right-hand side swept by the elementwise kernels (nE, or
@@ -132,7 +138,7 @@ void launch_stage_res64(const KArgs<double> &a, int nrhs, cudaStream_t s);
 // tensor maps of the input vectors, of sigma and of the signed node weights
 struct TmaMaps;
 int tma_maps_build(TmaMaps *m, const float2 *x0, const float2 *ph, const float2 *sh, const float2 *pw,
-                   const float2 *sw, const float *sig, const float *gdn, PadLayout pl, int nrhs);
+                   const float2 *sw, const float *sig, const float *gdn, PadLayout pl, PadLayout sl, int nrhs);
 TmaMaps *tma_maps_new();
 void tma_maps_free(TmaMaps *m);
 void launch_tma_init(const KArgs<float> &a, const TmaMaps *m, int nrhs, cudaStream_t s);

@@ -284,14 +284,15 @@ int Solver::update_cond(const double *m_earth, double airCond)
                       sigs32_.as<float>(), gdw32_.as<float>(), gdn32_.as<float>(), stream_);
     // sigma of both formulations and the signed node weights on the padded
     // layout (FP32), for the TMA-staged kernels
-    const size_t pe = (size_t)pl_.len(), pn = (size_t)pl_.Px * pl_.Py * pl_.Pz;
+    const PadLayout sl = sig_layout(pl_, nx);
+    const size_t pe = (size_t)sl.len(), pn = (size_t)pl_.Px * pl_.Py * pl_.Pz;
     if (sigP32_.alloc(pe * sizeof(float)) || sigsP32_.alloc(pe * sizeof(float)) || gdnP32_.alloc(pn * sizeof(float)))
         return fail(8, "mt3d_update_cond: out of device memory");
     cudaMemsetAsync(sigP32_.as<void>(), 0, pe * sizeof(float), stream_);
     cudaMemsetAsync(sigsP32_.as<void>(), 0, pe * sizeof(float), stream_);
     cudaMemsetAsync(gdnP32_.as<void>(), 0, pn * sizeof(float), stream_);
-    launch_to_padded(g64_, sig64_.as<double>(), pl_, sigP32_.as<float>(), stream_);
-    launch_to_padded(g64_, sigs64_.as<double>(), pl_, sigsP32_.as<float>(), stream_);
+    launch_to_padded(g64_, sig64_.as<double>(), sl, sigP32_.as<float>() + 1, stream_);
+    launch_to_padded(g64_, sigs64_.as<double>(), sl, sigsP32_.as<float>() + 1, stream_);
     launch_nodes_to_padded(g64_, gdn64_.as<double>(), pl_, gdnP32_.as<float>(), stream_);
     tma_stale_ = true;
     if ((rc = sync("mt3d_update_cond"))) return rc;
@@ -324,7 +325,7 @@ int Solver::tma_ready()
     Workspace &w = ws_;
     if (tma_maps_build(tma_, w.f_x0.as<float2>(), w.f_ph.as<float2>(), w.f_sh.as<float2>(), w.f_p.as<float2>(),
                        w.f_s.as<float2>(),
-                       (ctl.formulation == 1 ? sigsP32_ : sigP32_).as<float>(), gdnP32_.as<float>(), pl_, w.nrhs))
+                       (ctl.formulation == 1 ? sigsP32_ : sigP32_).as<float>(), gdnP32_.as<float>(), pl_, sig_layout(pl_, nx), w.nrhs))
         return fail(4, "cuTensorMapEncodeTiled failed for the padded FP32 vectors");
     tma_stale_ = false;
     return 0;
@@ -434,7 +435,8 @@ int Solver::ensure_workspace(int nrhs, int precision)
     int c;
     const ColMapHost cm = col_map(nx, ny);
     // partial sums: the stencil launches have up to one chunk per node plane
-    const int nb = std::max({blocks_for(nE, c), blocks_for(nN, c), cm.tiles * (nz + 1), 1184});
+    const int nb = std::max({blocks_for(nE, c), blocks_for(nN, c),
+                             std::max(cm.tiles, hat_map(nx, ny).tiles) * (nz + 1), 1184});
     err |= w.bst.alloc(nrhs * sizeof(BicgState)) | w.pst.alloc(nrhs * sizeof(PcgState)) |
            w.ost.alloc(nrhs * sizeof(OuterState)) | w.qst.alloc(nrhs * sizeof(QmrState));
     err |= w.parts.alloc((size_t)nrhs * nb * kMaxParts * sizeof(double)) | w.cnt.alloc(3 * nrhs * sizeof(unsigned));
@@ -540,6 +542,7 @@ template <> KArgs<float> Solver::kargs<float>(int nrhs, int)
     a.dsgn = -1.0;
     a.colstencil = w.padded ? 3 : 2;
     a.cmap = col_map(nx, ny);
+    a.hmap = hat_map(nx, ny);
     a.jinv = ctl.solver == 1 ? w.jinv32.as<float2>() : nullptr;
     if (ctl.formulation == 1) {
         a.sigma = sigs32_.as<float>();

@@ -169,32 +169,30 @@ template <typename K> static int stage_setup(K kern, size_t smem, int slot)
 
 // Time of a launch of c chunks of len planes (the last of them shorter) over
 // `layer` blocks each, in planes of a block that has its SM to itself.  A block
-// costs two planes to start; blocks that share an SM slow each other down by a
-// fifth each (the fused FP32 stencil: 1.55, 1.85, 2.2 and 2.5 us a plane with
-// one to four blocks, which is latency more than throughput, so a small grid
-// is faster in many short chunks than in few long ones).
+// costs a plane and a half to start; each further block on an SM slows all of
+// them down by a fifth (the fused FP32 stencil: 1.55, 1.85, 2.2 and 2.5 us a
+// plane with one to four blocks, so latency counts for more than throughput).
+// Full waves come first; the blocks of the last chunk fill the slots that the
+// others leave, as work that can be shared out, and a quarter of one at the end.
 static double stage_time(long layer, int c, int len, int last, long resident)
 {
     const auto shared = [](long blocks) { return 1.0 + 0.2 * ((blocks + 147) / 148 - 1); };
-    const long L = len + 2, l = last + 2, full = layer * (c - 1);
+    const double L = len + 1.5, l = last + 1.5;
     if (layer * c <= resident) return L * shared(layer * c);
-    const long r = full % resident, free_ = resident - r;
-    const double t = (double)(full / resident) * L * shared(resident);
-    if (r == 0) return t + (double)((layer + resident - 1) / resident) * l * shared(std::min(layer, resident));
-    // the short chunks go beside the last r of the others, and what is left after them
-    const long room = free_ * std::max<long>(1, L / l);
-    const long tail = layer <= room ? std::max(L, (layer + free_ - 1) / free_ * l)
-                                    : L + (layer - room + resident - 1) / resident * l;
-    return t + tail * shared(std::min(resident, r + layer));
+    const long full = layer * (c - 1), r = full % resident;
+    const double tail = std::max(r ? L : l, (r * L + layer * l) / resident + 0.25 * l);
+    return (double)(full / resident) * L * shared(resident) + tail * shared(std::min(resident, r + layer));
 }
 
 // chunks of node planes of a stencil launch over nrhs right-hand sides on a
 // GPU that holds `resident` blocks.  The blocks of right-hand sides that have
-// converged exit at once, so the choice weighs the launch with all, half and
-// one of them running.  us a launch of the fused FP32 stencil, against the
-// count for one right-hand side in chunks of at least 8 planes: 24^3 cells, 2
-// right-hand sides 11.6 (23.2); 40^3, 2: 16.2 (23.7); 64 x 64 x 48, 2: 24.4
-// (30.6); 100 x 100 x 60, 2: 48.7 (55.9); 200 x 200 x 100, 1: the same 3 chunks.
+// converged exit at once, so half and one of them running count a quarter each
+// beside all running.  Against the best of all counts measured over 24^3 to
+// 200 x 200 x 100 cells and 1 to 8 right-hand sides the choice takes 1.3 % more
+// time for the fused FP32 stencil and 1.0 % for the FP64 one (mean; 7 % at
+// most), and 8 % with half of them left; one count for a single right-hand side
+// in chunks of at least 8 planes took 22.3 instead of 10.9 us a launch on 24^3
+// cells with 2 right-hand sides.
 int stage_chunks(int nz, int tiles, int resident, int nrhs)
 {
     struct Last {
@@ -208,8 +206,8 @@ int stage_chunks(int nz, int tiles, int resident, int nrhs)
     for (int len = planes; len >= 1; len--) {
         const int c = (planes + len - 1) / len, last = planes - (c - 1) * len;
         if ((planes + c - 1) / c != len) continue;  // the same count in more even chunks comes later
-        double t = 0.0;
-        for (int n : {nrhs, (nrhs + 1) / 2, 1}) t += stage_time((long)n * tiles, c, len, last, resident);
+        const auto time = [&](int n) { return stage_time((long)n * tiles, c, len, last, resident); };
+        const double t = time(nrhs) + 0.25 * (time((nrhs + 1) / 2) + time(1));
         if (t < best_t - 1e-9) { best_t = t; best = c; }
     }
     memo = Last{nz, tiles, resident, nrhs, best};
@@ -218,7 +216,25 @@ int stage_chunks(int nz, int tiles, int resident, int nrhs)
 
 template <typename T> static dim3 stage_grid(const KArgs<T> &a, int nrhs, int resident)
 {
-    return dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, resident, nrhs));
+    // without the grad-div term a solve ends with the iteration's own residual
+    // (FWDsolve3D and its divergence correction), which other sums leave a few
+    // per cent from the true one: there the sums keep the order of the count for
+    // one right-hand side in chunks of at least 8 planes
+    int c = 1;
+    if (a.gd) {
+        c = stage_chunks(a.g.nz, a.cmap.tiles, resident, nrhs);
+    } else {
+        const int planes = a.g.nz + 1;
+        long best = LONG_MAX;
+        for (int q = 1; q <= std::max(1, planes / 8); q++) {
+            const long t = ((long)a.cmap.tiles * q + resident - 1) / resident * ((planes + q - 1) / q + 3);
+            if (t < best) {
+                best = t;
+                c = q;
+            }
+        }
+    }
+    return dim3(a.cmap.tiles, nrhs, c);
 }
 
 template <typename T> void launch_stage_init(const KArgs<T> &a, int nrhs, cudaStream_t s)

@@ -32,6 +32,10 @@
 
 namespace mt3d {
 
+constexpr int kTX = KctTile::TX, kTY = KctTile::TY, kFW = KctTile::FW, kFR = KctTile::FR, kSW = KctTile::SW,
+              kNW = KctTile::NW, kNR = KctTile::NR, kPhX = KctTile::PhX;
+constexpr unsigned kFBytes = KctTile::FBytes, kSBytes = KctTile::SBytes, kNBytes = KctTile::NBytes;
+
 extern std::atomic<long long> g_launch_count;
 static inline void counted(int n) { g_launch_count.fetch_add(n, std::memory_order_relaxed); }
 
@@ -40,7 +44,7 @@ static inline void counted(int n) { g_launch_count.fetch_add(n, std::memory_orde
 // existing edge of the thread's node column; e indexes the padded layout.
 // Returns false (all threads of the block alike) when a wait gave up.
 template <typename F>
-__device__ __forceinline__ bool tma_march(TmaSmem &sm, const TmaParams &tp, const Geo<float> &g, PadLayout pl,
+__device__ __forceinline__ bool tma_march(KctTile::Smem &sm, const TmaParams &tp, const Geo<float> &g, PadLayout pl,
                                           int r, const float2 *__restrict__ aux, bool gd, float wmu, int i0, int j0,
                                           int k0, int k1, int *err, int limit, F &&f)
 {
@@ -49,7 +53,7 @@ __device__ __forceinline__ bool tma_march(TmaSmem &sm, const TmaParams &tp, cons
     const bool live = i <= g.nx && j <= g.ny;
     const ColGeo<float> cg = col_geo(g, min(i, g.nx), min(j, g.ny));
     const int hf = (ty + 1) * kFW + tx + 2;  // own column in a field plane of the tile
-    const int hs = (ty + 1) * kSW + tx + 4;  // own column in a sigma plane
+    const int hs = (ty + 1) * kSW + tx + 1;  // own column in a sigma plane
     const int hn = ty * kPhX + tx;           // own node in a potential plane
     const int cf = kFR * kFW, cs = kFR * kSW;
     const int pxy = pl.Px * pl.Py, pc = pl.Pz * pxy;
@@ -88,7 +92,7 @@ __device__ __forceinline__ bool tma_march(TmaSmem &sm, const TmaParams &tp, cons
         const unsigned mb = smem_addr(&sm.mbar[s]);
         mbar_expect(mb, tx_bytes + (node ? kNBytes : 0u));
         tma_load4(smem_addr(sm.fld[s]), &tp.in, 2 * (i0 - 2), j0 - 1, p, 3 * r, mb);
-        tma_load4(smem_addr(sm.sig[mod3(p)]), &tp.sig, i0 - 4, j0 - 1, p, 0, mb);
+        tma_load4(smem_addr(sm.sig[mod3(p)]), &tp.sig, i0, j0 - 1, p, 0, mb);
         if (node) tma_load3(smem_addr(sm.nod[p & 1]), &tp.node, i0, j0, p, mb);
     };
     // this thread's bounded wait for the copies of plane p
@@ -111,8 +115,8 @@ __device__ __forceinline__ bool tma_march(TmaSmem &sm, const TmaParams &tp, cons
     };
     auto phi_plane = [&](int p) {
         const float dZ = (p >= 0 && p <= g.nz) ? g.delZ[p] : 0.f;
-        sm.phi[p & 1][hn] = tma_phi_node(sm, g, i, j, p, tx, ty, cg.delXi, cg.delYj, dZ);
-        if (hasH) sm.phi[p & 1][hnj * kPhX + hni] = tma_phi_node(sm, g, hi, hj, p, hni, hnj, hdX, hdY, dZ);
+        sm.phi[p & 1][hn] = tma_phi_node<KctTile>(sm, g, i, j, p, tx, ty, cg.delXi, cg.delYj, dZ);
+        if (hasH) sm.phi[p & 1][hnj * kPhX + hni] = tma_phi_node<KctTile>(sm, g, hi, hj, p, hni, hnj, hdX, hdY, dZ);
     };
     const float2 zero = make_float2(0.f, 0.f);
     float2 ax = zero, ay = zero, az = zero;
@@ -240,13 +244,13 @@ __global__ void __launch_bounds__(kThreads, 4) kct_init(const __grid_constant__ 
     if (!a.ost[r].active) return;
     BicgState &st = a.st[r];
     int i0, j0, k0, k1;
-    tma_tile(a.cmap, i0, j0);
-    tma_range(a.g.nz, k0, k1);
+    tma_tile_at<KctTile>(a.cmap, blockIdx.x, i0, j0);
+    tma_range_at(a.g.nz, blockIdx.z, gridDim.z, k0, k1);
     const size_t off = (size_t)r * a.stride;
     const float2 *b = a.b + off;
     float2 *R = a.r + off, *RT = a.rt + off;
     double u[2] = {0.0, 0.0};
-    const bool ok = tma_march(tma_smem(), tp, a.g, a.pl, r, b, a.gd != 0, (float)(a.dsgn * a.ost[r].omega * kMu0),
+    const bool ok = tma_march(tma_smem<KctTile>(), tp, a.g, a.pl, r, b, a.gd != 0, (float)(a.dsgn * a.ost[r].omega * kMu0),
                               i0, j0, k0, k1, a.err, a.wait_limit, [&](int, int e, bool in, float2 ax, float2, float2 bb) {
                                   float2 res = make_float2(0.f, 0.f);
                                   if (in) {
@@ -273,13 +277,13 @@ __global__ void __launch_bounds__(kThreads, 4) kct_vt(const __grid_constant__ Tm
     if (st.status != KS_RUNNING || !a.ost[r].active) return;
     if (a.sweeps && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.z == 0) atomicAdd(a.sweeps, 1ULL);
     int i0, j0, k0, k1;
-    tma_tile(a.cmap, i0, j0);
-    tma_range(a.g.nz, k0, k1);
+    tma_tile_at<KctTile>(a.cmap, blockIdx.x, i0, j0);
+    tma_range_at(a.g.nz, blockIdx.z, gridDim.z, k0, k1);
     const size_t off = (size_t)r * a.stride;
     const float2 *w = (which ? a.s : a.rt) + off;
     float2 *out = (which ? a.t : a.v) + off;
     double u[3] = {0.0, 0.0, 0.0};
-    const bool ok = tma_march(tma_smem(), tp, a.g, a.pl, r, w, a.gd != 0, (float)(a.dsgn * a.ost[r].omega * kMu0),
+    const bool ok = tma_march(tma_smem<KctTile>(), tp, a.g, a.pl, r, w, a.gd != 0, (float)(a.dsgn * a.ost[r].omega * kMu0),
                               i0, j0, k0, k1, a.err, a.wait_limit, [&](int, int e, bool inn, float2 y, float2, float2 q) {
                                   if (inn) {
                                       if (which == 0) {
@@ -341,24 +345,27 @@ TmaMaps *tma_maps_new()
 void tma_maps_free(TmaMaps *m) { delete m; }
 
 int tma_maps_build(TmaMaps *m, const float2 *x0, const float2 *ph, const float2 *sh, const float2 *pw,
-                   const float2 *sw, const float *sig, const float *gdn, PadLayout pl, int nrhs)
+                   const float2 *sw, const float *sig, const float *gdn, PadLayout pl, PadLayout sl, int nrhs)
 {
     m->ok = 0;
-    const cuuint64_t Px = pl.Px, Py = pl.Py, Pz = pl.Pz;
+    const cuuint64_t Px = pl.Px, Py = pl.Py, Pz = pl.Pz, Ps = sl.Px;
     // vectors: floats [nrhs * 3][Pz][Py][2 Px]
     const cuuint64_t vd[4] = {2 * Px, Py, Pz, 3 * (cuuint64_t)nrhs};
     const cuuint64_t vs[3] = {2 * Px * 4, 2 * Px * Py * 4, 2 * Px * Py * Pz * 4};
-    const cuuint32_t vb[4] = {2 * kFW, kFR, 1, 3};
-    // sigma: floats [3][Pz][Py][Px]; node weights: floats [Pz][Py][Px]
-    const cuuint64_t sd[4] = {Px, Py, Pz, 3};
-    const cuuint64_t ss[3] = {Px * 4, Px * Py * 4, Px * Py * Pz * 4};
-    const cuuint32_t sb[4] = {kSW, kFR, 1, 3};
+    // sigma: floats [3][Pz][Py][Ps]; node weights: floats [Pz][Py][Px]
+    const cuuint64_t sd[4] = {Ps, Py, Pz, 3};
+    const cuuint64_t ss[3] = {Ps * 4, Ps * Py * 4, Ps * Py * Pz * 4};
     const cuuint64_t nd[3] = {Px, Py, Pz};
     const cuuint64_t ns[2] = {Px * 4, Px * Py * 4};
-    const cuuint32_t nb[3] = {kNW, kNR, 1};
+    const cuuint32_t vb[4] = {2 * kFW, kFR, 1, 3}, sb[4] = {kSW, kFR, 1, 3}, nb[3] = {kNW, kNR, 1};
+    using H = HatTile;
+    const cuuint32_t hv[4] = {2 * H::FW, H::FR, 1, 3}, hs[4] = {H::SW, H::FR, 1, 3}, hn[3] = {H::NW, H::NR, 1};
+    if (!gdn) gdn = sig;
     if (encode(&m->x0, x0, 4, vd, vs, vb) || encode(&m->ph, ph, 4, vd, vs, vb) || encode(&m->sh, sh, 4, vd, vs, vb) ||
-        encode(&m->pw, pw, 4, vd, vs, vb) || encode(&m->sw, sw, 4, vd, vs, vb) ||
-        encode(&m->sig, sig, 4, sd, ss, sb) || encode(&m->node, gdn ? gdn : sig, 3, nd, ns, nb))
+        encode(&m->sig, sig, 4, sd, ss, sb) || encode(&m->node, gdn, 3, nd, ns, nb) ||
+        encode(&m->hx0, x0, 4, vd, vs, hv) || encode(&m->hph, ph, 4, vd, vs, hv) || encode(&m->hsh, sh, 4, vd, vs, hv) ||
+        encode(&m->hpw, pw, 4, vd, vs, hv) || encode(&m->hsw, sw, 4, vd, vs, hv) ||
+        encode(&m->hsig, sig, 4, sd, ss, hs) || encode(&m->hnode, gdn, 3, nd, ns, hn))
         return 1;
     m->ok = 1;
     return 0;
@@ -371,7 +378,7 @@ void launch_tma_init(const KArgs<float> &a, const TmaMaps *m, int nrhs, cudaStre
     tp.in = m->x0;
     tp.sig = m->sig;
     tp.node = m->node;
-    const size_t sm = sizeof(TmaSmem);
+    const size_t sm = sizeof(KctTile::Smem);
     const int res = tma_resident(kct_init, sm, 0);
     kct_init<<<dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kThreads, sm, s>>>(tp, a);
 }
@@ -382,7 +389,7 @@ void launch_tma_vt(const KArgs<float> &a, const TmaMaps *m, int which, int nrhs,
     tp.in = which ? m->sh : m->ph;
     tp.sig = m->sig;
     tp.node = m->node;
-    const size_t sm = sizeof(TmaSmem);
+    const size_t sm = sizeof(KctTile::Smem);
     const int res = tma_resident(kct_vt, sm, 1);
     kct_vt<<<dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kThreads, sm, s>>>(tp, a, which);
 }

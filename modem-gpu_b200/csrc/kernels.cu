@@ -219,6 +219,7 @@ template <typename T> __global__ void __launch_bounds__(kThreads) kb_init(KArgs<
 // p = r (first iteration) or p = r + beta (p - omega v); ph = M^-1 p
 template <typename T> __global__ void __launch_bounds__(kThreads) kb_p(KArgs<T> a)
 {
+    launch_wait();
     const int r = blockIdx.y;
     const BicgState &st = a.st[r];
     if (st.status != KS_RUNNING || !a.ost[r].active) return;
@@ -287,6 +288,7 @@ template <typename T> __global__ void __launch_bounds__(kThreads) kb_v(KArgs<T> 
 // s = r - alpha v ; sh = M^-1 s
 template <typename T> __global__ void __launch_bounds__(kThreads) kb_s(KArgs<T> a)
 {
+    launch_wait();
     const int r = blockIdx.y;
     const BicgState &st = a.st[r];
     if (st.status != KS_RUNNING || !a.ost[r].active) return;
@@ -348,6 +350,7 @@ template <typename T> __global__ void __launch_bounds__(kThreads) kb_t(KArgs<T> 
 // beta for the next iteration
 template <typename T> __global__ void __launch_bounds__(kThreads) kb_xr(KArgs<T> a)
 {
+    launch_wait();
     const int r = blockIdx.y;
     BicgState &st = a.st[r];
     if (st.status != KS_RUNNING || !a.ost[r].active) return;
@@ -1445,7 +1448,7 @@ void launch_bicg_iter(const KArgs<T> &a, int nrhs, cudaStream_t s, cudaEvent_t *
     counted(a.colstencil ? 3 : 5);
     dim3 grid(a.nblk, nrhs);
     const bool staged = a.colstencil >= 2;
-    kb_p<T><<<grid, kThreads, 0, s>>>(a);
+    launch_chained(kb_p<T>, grid, kThreads, 0, s, a);
     if (pc) launch_col_prec(*pc, a.p, a.ph, nrhs, s);
     if (a.gd && !staged) launch_gd_phi(a, a.ph, a.phi, 0, nrhs, s);
     if (ev) cudaEventRecord(ev[0], s);
@@ -1455,7 +1458,7 @@ void launch_bicg_iter(const KArgs<T> &a, int nrhs, cudaStream_t s, cudaEvent_t *
     else if (a.colstencil) launch_colb_vt(a, 0, nrhs, s);
     else kb_v<T><<<grid, kThreads, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[1], s);
-    kb_s<T><<<grid, kThreads, 0, s>>>(a);
+    launch_chained(kb_s<T>, grid, kThreads, 0, s, a);
     if (pc) launch_col_prec(*pc, a.s, a.sh, nrhs, s);
     if (a.gd && !staged) launch_gd_phi(a, a.sh, a.phi, 0, nrhs, s);
     if (ev) cudaEventRecord(ev[2], s);
@@ -1465,7 +1468,7 @@ void launch_bicg_iter(const KArgs<T> &a, int nrhs, cudaStream_t s, cudaEvent_t *
     else if (a.colstencil) launch_colb_vt(a, 1, nrhs, s);
     else kb_t<T><<<grid, kThreads, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[3], s);
-    kb_xr<T><<<grid, kThreads, 0, s>>>(a);
+    launch_chained(kb_xr<T>, grid, kThreads, 0, s, a);
 }
 template <typename T> void launch_bicg_finish(const KArgs<T> &a, int nrhs, cudaStream_t s)
 {

@@ -76,6 +76,7 @@ template <typename T> __global__ void __launch_bounds__(kThreads, sizeof(T) == 4
 // t = A sh ; ts = t . s, tt = t . t ; omega     (which = 1)
 template <typename T> __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 4 : 2) kcs_vt(KArgs<T> a, int which)
 {
+    launch_wait();
     const int r = blockIdx.y;
     BicgState &st = a.st[r];
     if (st.status != KS_RUNNING || !a.ost[r].active) return;
@@ -249,7 +250,7 @@ template <typename T> void launch_stage_vt(const KArgs<T> &a, int which, int nrh
     counted(1);
     const size_t sm = sizeof(StageSmem<T>);
     const int res = stage_setup(kcs_vt<T>, sm, sizeof(T) == 8 ? 2 : 3);
-    kcs_vt<T><<<stage_grid(a, nrhs, res), kThreads, sm, s>>>(a, which);
+    launch_chained(kcs_vt<T>, stage_grid(a, nrhs, res), kThreads, sm, s, a, which);
 }
 void launch_stage_res64(const KArgs<double> &a, int nrhs, cudaStream_t s)
 {

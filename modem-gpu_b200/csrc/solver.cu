@@ -1084,6 +1084,15 @@ int Solver::solve_begin(SolveRun &run, int nrhs, const double *omegas, const int
     return 0;
 }
 
+// How far an FP32 cycle takes its own residual at most.  The iteration's
+// recursion goes on falling where FP32 can no longer lower the true residual
+// (some 1e-6 of the cycle's start), so a cycle that reaches this has nothing
+// left to gain and the next one goes on from the true residual.  Solves to 1e-12
+// on 19 grids of 24^3 to 200 x 200 x 100 cells took 6 % less time with 3e-7 (24^3:
+// 12.8 -> 9.4 ms), 5 % with 1e-7, 6 to 7 % with 1e-6 to 1e-5; solves to 1e-7 the
+// same to 1 % with all of them.
+constexpr double kInnerFloor = 3e-7;
+
 // start of an outer cycle: the true FP64 residual r64 = b - A X (into tmp);
 // converged right-hand sides leave the loop; the FP32 and FP64 groups of the
 // mixed-precision cycle; the FP32 group marked active on the device
@@ -1114,7 +1123,7 @@ int Solver::solve_pre(SolveRun &run)
             if (!std::isfinite(o.relres)) { o.active = 0; o.failed = 3; continue; }
             if (o.relres <= o.tol) { o.active = 0; o.converged = 1; continue; }
             if (o.nDivCor >= ctl.MaxDivCor) { o.active = 0; o.failed = 1; continue; }
-            o.tol_inner = o.tol * o.bnorm64 * o.scale;  // tol*||b|| relative to ||r64||
+            o.tol_inner = std::max(o.tol * o.bnorm64 * o.scale, kInnerFloor);  // tol*||b|| relative to ||r64||
             // an FP32 cycle that did not halve the true residual: when its
             // own iteration converged well, the FP32 operator's rounding is
             // the limit and the right-hand side moves to FP64; when the

@@ -928,9 +928,6 @@ int launch_hat_iter_multi(const KArgs<float> *args, const int *nrhs, const int *
     tma_resident(kh_vt_multi<4>, smb, 20, kHatThreads);
     tma_resident(kh_vt_multi<5>, smb, 21, kHatThreads);
     p.eb0[0] = p.sb0[0] = 0;
-    const auto planes_of = [&](int g) { return (double)nrhs[g] * args[g].hmap.tiles * (args[g].g.nz + 1); };
-    double all = 0.0;
-    for (int g = 0; g < ng; g++) all += planes_of(g);
     for (int g = 0; g < ng; g++) {
         p.a[g] = args[g];
         p.nr[g] = nrhs[g];
@@ -942,11 +939,11 @@ int launch_hat_iter_multi(const KArgs<float> *args, const int *nrhs, const int *
             p.tp[g][w].sig = args[g].tma->hsig;
             p.tp[g][w].node = args[g].tma->hnode;
         }
-        // a grid's share of the resident blocks is its share of the work; more
-        // chunks than planes would only add empty ones, and the reductions'
-        // partial sums have room for one chunk per plane
-        const int share = std::max(1, (int)(res * (planes_of(g) / all)));
-        p.zch[g] = std::min(zch && zch[g] > 0 ? zch[g] : stage_chunks(args[g].g.nz, args[g].hmap.tiles, share, nrhs[g]),
+        // the count of the grid by itself (the blocks of the grids mix, and the
+        // time is flat about it: 262 to 273 ms for 40^3 + 64 x 64 x 48 cells with
+        // counts from 3, 5 to 11, 13); more chunks than planes would only add
+        // empty ones, and the reductions' partial sums have room for one a plane
+        p.zch[g] = std::min(zch && zch[g] > 0 ? zch[g] : stage_chunks(args[g].g.nz, args[g].hmap.tiles, res, nrhs[g]),
                             args[g].g.nz + 1);
         p.eb0[g + 1] = p.eb0[g] + nrhs[g] * args[g].nblk;
         p.sb0[g + 1] = p.sb0[g] + nrhs[g] * args[g].hmap.tiles * p.zch[g];

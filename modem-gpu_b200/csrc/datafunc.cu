@@ -11,7 +11,7 @@
 // weights go up in one copy, and the scratch stays with the handle.  (Built
 // on the host with a linear search per coordinate, a sort of the entries by
 // edge and ten allocations, the adjoint sources of 400 sites on 100 x 100 x 60
-// cells took 1.97 ms; here 0.19 ms.)  Site azimuths are zero (the reference's
+// cells took 1.97 ms; here 0.09 ms.)  Site azimuths are zero (the reference's
 // rotate_Model2Data with zero angles).
 #include <algorithm>
 #include <cmath>
@@ -114,23 +114,18 @@ __device__ int min_node(double x, const double *c, int n)
     return lo;
 }
 
-// E lies on edges: centred along its own axis; B on faces: centred along the
+// Point before the site along axis a and the weight of the point after it.  E
+// lies on edges: centred along its own axis; B on faces: centred along the
 // other two (EinterpSetUp and BinterpSetUp without conductivity weighting)
-__device__ SiteFun site_fun(const SiteGrid &g, const double *x, int f)
+__device__ void site_axis(const SiteGrid &g, const double *x, int f, int a, int &p, double &w)
 {
-    SiteFun r;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const Axis &A = g.ax[a];
-        const bool centred = (a == (f & 1)) == (f < 2);
-        const double xc = clean(x[a]);
-        const int nmax = centred ? A.n : A.n + 1;
-        const int p = centred ? min_node(xc, A.ccentre, A.n) : min_node(xc, A.cnode, A.n + 1);
-        r.p[a] = p;
-        if (p > 0 && p < nmax) r.w[a] = centred ? (x[a] - A.centre[p - 1]) / A.del[p] : (x[a] - A.node[p - 1]) / A.d[p - 1];
-        else r.w[a] = p <= 0 ? 1.0 : 0.0;
-    }
-    return r;
+    const Axis &A = g.ax[a];
+    const bool centred = (a == (f & 1)) == (f < 2);
+    const double xc = clean(x[a]);
+    const int nmax = centred ? A.n : A.n + 1;
+    p = min_node(xc, centred ? A.ccentre : A.cnode, nmax);
+    if (p > 0 && p < nmax) w = centred ? (x[a] - A.centre[p - 1]) / A.del[p] : (x[a] - A.node[p - 1]) / A.d[p - 1];
+    else w = p <= 0 ? 1.0 : 0.0;
 }
 
 // flat 0-based edge index of 1-based (component, i, j, k); -1 outside the grid
@@ -188,54 +183,90 @@ __device__ bool site_term(const SiteGrid &g, const SiteFun &s, int f, int t, int
     im = c * w * g.ioi;
     return true;
 }
-__device__ __forceinline__ int site_terms(int f) { return f < 2 ? 8 : 32; }
-constexpr int kSiteTerms = 80;  // of the four functionals
-
-__device__ __forceinline__ cd shfl_cd(cd v, int src)
+// The terms of functional f that edge (c, i, j, k) can be: its one corner of E,
+// the two faces it bounds of B, in ascending order.
+__device__ int edge_terms(const SiteFun &s, int f, int c, int i, int j, int k, int (&t)[2])
 {
-    return {__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
+    const auto corner = [&](int I, int J, int K) {
+        const unsigned n = I - s.p[0], m = J - s.p[1], p = K - s.p[2];
+        return (n | m | p) > 1u ? -1 : (int)(4 * n + 2 * m + p);
+    };
+    int nt = 0;
+    if (f < 2) {
+        const int q = c == f + 1 ? corner(i, j, k) : -1;
+        if (q >= 0) t[nt++] = q;
+        return nt;
+    }
+    if (c == f - 1) return 0;  // Ex is on no x-face, Ey on no y-face
+    // the edge as the far side of the face before it, and as the near side
+    const bool vert = c == 3;
+    const int lo = !vert ? corner(i, j, k - 1) : f == 2 ? corner(i, j - 1, k) : corner(i - 1, j, k), hi = corner(i, j, k);
+    const int q = (f == 2) == vert ? 2 : 0;  // its pair of the face's four edges
+    if (lo >= 0) t[nt++] = 4 * lo + q + 1;
+    if (hi >= 0) t[nt++] = 4 * hi + q;
+    return nt;
 }
+__device__ __forceinline__ int site_terms(int f) { return f < 2 ? 8 : 32; }
+__device__ __forceinline__ int site_base(int f) { return f < 2 ? 8 * f : 32 * f - 48; }  // the terms before them
+constexpr int kSiteTerms = 80, kSiteBlock = 96;  // of the four functionals; threads for them
 
 }  // namespace
 
-// Four lanes per site, one functional each: the functionals on both
-// polarisations, Z and B^-1 (dataResp); with d non-null also the weights of
-// the four functionals in the adjoint source of each polarisation k (Lrows +
-// LmultT for Full_Impedance, f90/3D_MT/DataFunc.f90:465-869,
-// f90/SENS/DataSens.f90:130-225):
+// A warp per site.  Twelve lanes search the axes of the four functionals, then
+// the lanes take the terms of one functional after another and add them up in
+// a fixed tree: the functionals on both polarisations, Z and B^-1 (dataResp);
+// with d non-null also the weights of the four functionals in the adjoint
+// source of each polarisation k (Lrows + LmultT for Full_Impedance,
+// f90/3D_MT/DataFunc.f90:465-869, f90/SENS/DataSens.f90:130-225):
 //   s_k = sum_ij conj(d_ij) B^-1(k, j) (Le_i - Z_i1 Lbx - Z_i2 Lby)
-// err: the first site (+ 1) with an edge outside the grid.
-__global__ void __launch_bounds__(64) k_site(SiteGrid g, int nsite, const double *xyz, SiteFun *fun, const double2 *e1,
-                                             const double2 *e2, double2 *Z, const double2 *d, double2 *W, unsigned *err)
+// err: the first site (+ 1) with an edge outside the grid.  Bound by the
+// latency of the searches and gathers: 14 us for 400 sites; 34 us with four
+// lanes a site and its terms one after another.
+__global__ void __launch_bounds__(64) k_site(SiteGrid g, int nsite, const double *xyz, SiteFun *fun, int *lo,
+                                             const double2 *e1, const double2 *e2, double2 *Z, const double2 *d, double2 *W,
+                                             unsigned *err)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, f = t & 3;
-    const bool live = t >> 2 < nsite;
-    const int s = live ? t >> 2 : nsite - 1;  // (every lane takes part in the exchange)
-    const SiteFun sf = site_fun(g, xyz + 3 * (size_t)s, f);
-    if (live) fun[4 * (size_t)s + f] = sf;
-    cd a = {0.0, 0.0}, b = {0.0, 0.0};
-    for (int q = 0; q < site_terms(f); q++) {
+    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (s >= nsite) return;
+    int p = 0;
+    double w = 0.0;
+    if (lane < 12) site_axis(g, xyz + 3 * (size_t)s, lane / 3, lane % 3, p, w);
+    // the smallest of the functionals' points along each axis
+    int low = p;
+    for (int f = 1; f < 4; f++) low = min(low, __shfl_sync(0xffffffffu, p, (lane + 3 * f) % 12));
+    if (lane < 3) lo[3 * (size_t)s + lane] = low;
+    cd v[4][2];
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+        SiteFun sf;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            sf.p[a] = __shfl_sync(0xffffffffu, p, 3 * f + a);
+            sf.w[a] = __shfl_sync(0xffffffffu, w, 3 * f + a);
+        }
+        if (lane == f) fun[4 * (size_t)s + f] = sf;
+        double t[4] = {0.0, 0.0, 0.0, 0.0};
         int e;
         double re, im;
-        if (!site_term(g, sf, f, q, e, re, im)) continue;
-        if (e < 0) {
-            if (live) atomicMin(err, (unsigned)s + 1u);
-            continue;
+        if (lane < site_terms(f) && site_term(g, sf, f, lane, e, re, im)) {
+            if (e < 0) {
+                atomicMin(err, (unsigned)s + 1u);
+            } else {
+                const double2 x1 = e1[e], x2 = e2[e];
+                const cd a = cd_mul(cd{re, im}, cd{x1.x, x1.y}), b = cd_mul(cd{re, im}, cd{x2.x, x2.y});
+                t[0] = a.re;
+                t[1] = a.im;
+                t[2] = b.re;
+                t[3] = b.im;
+            }
         }
-        const cd c = {re, im};
-        const double2 x1 = e1[e], x2 = e2[e];
-        a = cd_add(a, cd_mul(c, cd{x1.x, x1.y}));
-        b = cd_add(b, cd_mul(c, cd{x2.x, x2.y}));
+        __syncwarp();
+        warp_sum<4>(t);
+        v[f][0] = {t[0], t[1]};
+        v[f][1] = {t[2], t[3]};
     }
-    __syncwarp();
-    cd v[4][2];
-    const int l0 = threadIdx.x & 28;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        v[q][0] = shfl_cd(a, l0 + q);
-        v[q][1] = shfl_cd(b, l0 + q);
-    }
-    if (!live) return;
+    if (lane >= 4) return;
+    const int f = lane;
     // EE(i, m) = v[i][m], BB(i, m) = v[2 + i][m]; BB^-1 by Kramer's rule
     const cd det = cd_sub(cd_mul(v[2][0], v[3][1]), cd_mul(v[2][1], v[3][0]));
     cd bi[2][2], z[2][2];
@@ -281,58 +312,67 @@ __global__ void __launch_bounds__(kThreads) k_site_clear(int nE, double2 *s1, do
 // Adjoint sources.  A block takes one site, a thread one of its terms; the
 // thread of the first term with an edge, in the order (site, functional, term),
 // adds every site's share of it in that order, the others leave: no atomics
-// and no sort, so sources are reproducible.  The search over the other sites
-// is a test of three integers each, of order nsite^2 in all: 400 sites a few
-// microseconds, 10 000 about two milliseconds.
-__global__ void __launch_bounds__(96) k_site_scatter(SiteGrid g, int nsite, const SiteFun *fun, const double2 *W,
-                                                     double2 *s1, double2 *s2, const unsigned *err)
+// and no sort, so sources are reproducible.  The block picks the sites nearby,
+// a test of three integers for each site by one thread, of order nsite^2 in
+// all, and such a site costs the few terms that the edge can be.  (All 80 terms
+// of a site tried and the sites tested by every thread: 94 us for 400 sites;
+// the few terms alone: 43 us; now 18 us.)
+__global__ void __launch_bounds__(kSiteBlock) k_site_scatter(SiteGrid g, int nsite, const SiteFun *fun, const int *lo,
+                                                             const double2 *W, double2 *s1, double2 *s2,
+                                                             const unsigned *err)
 {
-    constexpr int kTile = 512;
-    __shared__ int lo[kTile][3], own[kSiteTerms];
+    __shared__ int near[kSiteBlock], found[kSiteBlock / 32];
     if (*err != ~0u) return;
-    const int s = blockIdx.x, t = threadIdx.x;
+    const int s = blockIdx.x, t = threadIdx.x, lane = t & 31, wp = t >> 5;
     int e = -1;
     if (t < kSiteTerms) {
-        const int f = t < 8 ? 0 : t < 16 ? 1 : t < 48 ? 2 : 3, q = t - (f == 0 ? 0 : f == 1 ? 8 : f == 2 ? 16 : 48);
+        const int f = t < 8 ? 0 : t < 16 ? 1 : t < 48 ? 2 : 3;
         double re, im;
-        if (!site_term(g, fun[4 * (size_t)s + f], f, q, e, re, im)) e = -1;
-        own[t] = e;
+        if (!site_term(g, fun[4 * (size_t)s + f], f, t - site_base(f), e, re, im)) e = -1;
     }
-    __syncthreads();
     bool mine = e >= 0;
-    for (int q = 0; q < t && mine; q++) mine = own[q] != e;
-    // (i, j, k) of the edge, 1-based
-    int i = 0, j = 0, k = 0;
+    // component and (i, j, k) of the edge, 1-based
+    int c = 0, i = 0, j = 0, k = 0;
     if (mine) {
         const int nXe = g.nx * (g.ny + 1) * (g.nz + 1), nYe = (g.nx + 1) * g.ny * (g.nz + 1);
-        const int c = e < nXe ? 1 : e < nXe + nYe ? 2 : 3;
+        c = e < nXe ? 1 : e < nXe + nYe ? 2 : 3;
         const int r = e - (c == 1 ? 0 : c == 2 ? nXe : nXe + nYe), ni = c == 1 ? g.nx : g.nx + 1, nj = c == 2 ? g.ny : g.ny + 1;
         i = r % ni + 1;
         j = r / ni % nj + 1;
         k = r / (ni * nj) + 1;
     }
+    const int l0 = lo[3 * (size_t)s], l1 = lo[3 * (size_t)s + 1], l2 = lo[3 * (size_t)s + 2];
     cd a = {0, 0}, b = {0, 0};
-    for (int s0 = 0; s0 < nsite; s0 += kTile) {
+    for (int r0 = 0; r0 < nsite; r0 += kSiteBlock) {
         // a site's edges lie within three of its smallest indices: its points
         // differ by at most one between the functionals, a corner and a face's
         // far side add one each
+        bool hit = false;
+        if (r0 + t < nsite) {
+            const int *l = lo + 3 * (size_t)(r0 + t);
+            hit = abs(l[0] - l0) <= 3 && abs(l[1] - l1) <= 3 && abs(l[2] - l2) <= 3;
+        }
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (lane == 0) found[wp] = __popc(hits);
         __syncthreads();
-        for (int q = t; q < min(kTile, nsite - s0); q += blockDim.x)
-            for (int x = 0; x < 3; x++) {
-                const SiteFun *F = fun + 4 * (size_t)(s0 + q);
-                lo[q][x] = min(min(F[0].p[x], F[1].p[x]), min(F[2].p[x], F[3].p[x]));
-            }
+        int at = 0, all = 0;
+        for (int q = 0; q < kSiteBlock / 32; q++) {
+            at += q < wp ? found[q] : 0;
+            all += found[q];
+        }
+        if (hit) near[at + __popc(hits & ((1u << lane) - 1u))] = r0 + t;
         __syncthreads();
-        for (int q = 0; q < min(kTile, nsite - s0) && mine; q++) {
-            if ((unsigned)(i - lo[q][0]) > 3u || (unsigned)(j - lo[q][1]) > 3u || (unsigned)(k - lo[q][2]) > 3u) continue;
-            const int r = s0 + q;
+        for (int q = 0; q < all && mine; q++) {
+            const int r = near[q];
             for (int f = 0; f < 4 && mine; f++) {
+                int can[2];
                 const SiteFun sf = fun[4 * (size_t)r + f];
-                for (int u = 0; u < site_terms(f); u++) {
+                const int nt = edge_terms(sf, f, c, i, j, k, can);
+                for (int u = 0; u < nt; u++) {
                     int ee;
                     double re, im;
-                    if (!site_term(g, sf, f, u, ee, re, im) || ee != e) continue;
-                    if (r < s) {  // an earlier site has the edge
+                    if (!site_term(g, sf, f, can[u], ee, re, im) || ee != e) continue;
+                    if (r < s || (r == s && site_base(f) + can[u] < t)) {  // an earlier site or term has the edge
                         mine = false;
                         break;
                     }
@@ -342,6 +382,7 @@ __global__ void __launch_bounds__(96) k_site_scatter(SiteGrid g, int nsite, cons
                 }
             }
         }
+        __syncthreads();
     }
     if (!mine) return;
     s1[e] = make_double2(a.re, a.im);
@@ -391,22 +432,29 @@ int Solver::data_functional(double om, int nsite, const double *xyz, const doubl
     if (d) up.insert(up.end(), d, d + 8 * (size_t)nsite);
     const size_t ox = up.size();
     up.insert(up.end(), xyz, xyz + 3 * (size_t)nsite);
-    // scratch of the handle: those, the functionals, W, Z and the error word
+    // the error word, set to none; the impedances follow it, for one copy down
+    if (up.size() & 1) up.push_back(0.0);
+    const size_t oe = up.size();
+    up.resize(oe + 2);
+    std::memset(&up[oe], 0xff, 2 * sizeof(double));
+    // scratch of the handle: those, the impedances, the functionals, W and the smallest indices
     const size_t eb = (size_t)nE * sizeof(double2), ns = (size_t)nsite;
     const auto align = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t b0 = align(up.size() * sizeof(double)), b1 = align(4 * ns * sizeof(SiteFun)),
-                 b2 = align(8 * ns * sizeof(double2)), b3 = align(4 * ns * sizeof(double2));
+    const size_t bz = Zout ? 4 * ns * sizeof(double2) : 0;
+    const size_t b0 = align(up.size() * sizeof(double) + bz), b1 = align(4 * ns * sizeof(SiteFun)),
+                 b2 = align(d ? 8 * ns * sizeof(double2) : 0), b3 = 3 * ns * sizeof(int);
     DevBuf de1, de2, ds1, ds2;
-    if (site_.alloc(b0 + b1 + b2 + b3 + sizeof(unsigned)) || (!device && (de1.alloc(eb) || de2.alloc(eb))) ||
+    if (site_.alloc(b0 + b1 + b2 + b3) || (!device && (de1.alloc(eb) || de2.alloc(eb))) ||
         (!device && d && (ds1.alloc(eb) || ds2.alloc(eb))))
         return fail(8, std::string(who) + ": out of device memory");
     unsigned char *base = site_.as<unsigned char>();
     const double *tab = reinterpret_cast<const double *>(base);
+    unsigned *err = reinterpret_cast<unsigned *>(base + oe * sizeof(double));
+    double2 *dz = reinterpret_cast<double2 *>(base + up.size() * sizeof(double));
     SiteFun *fun = reinterpret_cast<SiteFun *>(base + b0);
-    double2 *W = reinterpret_cast<double2 *>(base + b0 + b1), *dz = reinterpret_cast<double2 *>(base + b0 + b1 + b2);
-    unsigned *err = reinterpret_cast<unsigned *>(base + b0 + b1 + b2 + b3);
+    double2 *W = reinterpret_cast<double2 *>(base + b0 + b1);
+    int *lo = reinterpret_cast<int *>(base + b0 + b1 + b2);
     cudaMemcpyAsync(base, up.data(), up.size() * sizeof(double), cudaMemcpyHostToDevice, stream_);
-    cudaMemsetAsync(err, 0xff, sizeof(unsigned), stream_);
     SiteGrid g;
     g.nx = nx;
     g.ny = ny;
@@ -423,25 +471,23 @@ int Solver::data_functional(double om, int nsite, const double *xyz, const doubl
         p2 = de2.as<double2>();
     }
     g_launch_count.fetch_add(d ? 3 : 1, std::memory_order_relaxed);
-    k_site<<<(4 * nsite + 63) / 64, 64, 0, stream_>>>(g, nsite, tab + ox, fun, p1, p2, Zout ? dz : nullptr,
-                                                      d ? reinterpret_cast<const double2 *>(tab + od) : nullptr,
-                                                      d ? W : nullptr, err);
+    k_site<<<(nsite + 1) / 2, 64, 0, stream_>>>(g, nsite, tab + ox, fun, lo, p1, p2, Zout ? dz : nullptr,
+                                                  d ? reinterpret_cast<const double2 *>(tab + od) : nullptr, d ? W : nullptr,
+                                                  err);
     double2 *q1 = nullptr, *q2 = nullptr;
     if (d) {
         q1 = device ? reinterpret_cast<double2 *>(s1) : ds1.as<double2>();
         q2 = device ? reinterpret_cast<double2 *>(s2) : ds2.as<double2>();
         k_site_clear<<<148 * 8, kThreads, 0, stream_>>>((int)nE, q1, q2, err);
-        k_site_scatter<<<nsite, 96, 0, stream_>>>(g, nsite, fun, W, q1, q2, err);
+        k_site_scatter<<<nsite, kSiteBlock, 0, stream_>>>(g, nsite, fun, lo, W, q1, q2, err);
     }
-    // impedances and the error word, which follow one another, in one copy down
-    const size_t bz = Zout ? b3 : 0;
-    std::vector<unsigned char> down(bz + sizeof(unsigned));
-    cudaMemcpyAsync(down.data(), reinterpret_cast<unsigned char *>(err) - bz, down.size(), cudaMemcpyDeviceToHost, stream_);
+    std::vector<unsigned char> down(2 * sizeof(double) + bz);
+    cudaMemcpyAsync(down.data(), err, down.size(), cudaMemcpyDeviceToHost, stream_);
     if (int rc = sync(who)) return rc;
     unsigned bad;
-    std::memcpy(&bad, down.data() + bz, sizeof bad);
+    std::memcpy(&bad, down.data(), sizeof bad);
     if (bad != ~0u) return fail(5, std::string(who) + ": site " + std::to_string(bad - 1) + " needs an edge outside the grid");
-    if (Zout) std::memcpy(Zout, down.data(), 4 * ns * sizeof(double2));
+    if (Zout) std::memcpy(Zout, down.data() + 2 * sizeof(double), bz);
     if (!d || device) return 0;
     cudaMemcpyAsync(s1, q1, eb, cudaMemcpyDeviceToHost, stream_);
     cudaMemcpyAsync(s2, q2, eb, cudaMemcpyDeviceToHost, stream_);

@@ -57,35 +57,53 @@ constexpr unsigned kFBytes = HatTile::FBytes, kSBytes = HatTile::SBytes, kNBytes
 extern std::atomic<long long> g_launch_count;
 static inline void counted(int n) { g_launch_count.fetch_add(n, std::memory_order_relaxed); }
 
-// diagonal of A at an interior edge: dr + i di
-__device__ __forceinline__ void hat_diag(int comp, const ColGeo<float> &cg, const PlaneGeo<float> &pg, float wmu,
-                                         float sig, bool gd, float wns, float wne, float &dr, float &di)
+// diagonal dr + i di of A at an interior edge: the curl-curl part p sp + q sq
+// (p, q: the weights of the curls beside the edge; sp, sq: the sums of 1 / d of
+// the two cells across each), the grad-div part a^2 (w_s c_s + w_e c_e) with a
+// the dual face's area and c = sigma at earth nodes (negative weights), one in
+// the air, and di = v sigma with v = omega mu0 V_E.  The roundings are written
+// out, so that every kernel has the same D.
+__device__ __forceinline__ void hat_diag(float p, float sp, float q, float sq, float v, float sig, bool gd, float a,
+                                         float ws, float we, float &dr, float &di)
 {
-    float ve, dfa;
-    if (comp == 0) {
-        ve = cg.dxi * (cg.delYj * pg.delZk);
-        dfa = cg.delYj * pg.delZk;
-    } else if (comp == 1) {
-        ve = cg.dyj * (cg.delXi * pg.delZk);
-        dfa = cg.delXi * pg.delZk;
-    } else {
-        ve = pg.dzk * (cg.delXi * cg.delYj);
-        dfa = cg.delXi * cg.delYj;
-    }
-    dr = col_ccdiag(comp, cg, pg);
+    dr = __fmaf_rn(p, sp, __fmul_rn(q, sq));
     if (gd) {
-        const float cs = wns < 0.f ? sig : 1.f, ce = wne < 0.f ? sig : 1.f;
-        dr += dfa * dfa * (fabsf(wns) * cs + fabsf(wne) * ce);
+        const float n = __fadd_rn(fmaxf(ws, __fmul_rn(-ws, sig)), fmaxf(we, __fmul_rn(-we, sig)));
+        dr = __fmaf_rn(__fmul_rn(a, a), n, dr);
     }
-    di = wmu * sig * ve;
+    di = __fmul_rn(v, sig);
+}
+// what a plane gives a node's edges: the weights of the curls beside Ex, Ey and
+// Ez (dxi delZk, dxi delYj; dyj delXi, dyj delZk; dzk delYj, dzk delXi), and the
+// areas of their dual faces
+struct HatCoef {
+    float xz, xy, yx, yz, zy, zx, ax, ay, az;
+};
+__device__ __forceinline__ HatCoef hat_coef(const ColGeo<float> &c, const PlaneGeo<float> &p)
+{
+    return {__fmul_rn(c.dxi, p.delZk),   __fmul_rn(c.dxi, c.delYj),   __fmul_rn(c.dyj, c.delXi),
+            __fmul_rn(c.dyj, p.delZk),   __fmul_rn(p.dzk, c.delYj),   __fmul_rn(p.dzk, c.delXi),
+            __fmul_rn(c.delYj, p.delZk), __fmul_rn(c.delXi, p.delZk), __fmul_rn(c.delXi, c.delYj)};
+}
+__device__ __forceinline__ void hat_diag_of(int comp, const ColGeo<float> &c, const PlaneGeo<float> &p, const HatCoef &w,
+                                            float wmu, float sig, bool gd, float ws, float we, float &dr, float &di)
+{
+    const float sx = __fadd_rn(c.rdxi, c.rdxim1), sy = __fadd_rn(c.rdyj, c.rdyjm1), sz = __fadd_rn(p.rdzk, p.rdzkm1);
+    if (comp == 0) hat_diag(w.xz, sy, w.xy, sz, __fmul_rn(__fmul_rn(wmu, p.delZk), w.xy), sig, gd, w.ax, ws, we, dr, di);
+    else if (comp == 1) hat_diag(w.yz, sx, w.yx, sz, __fmul_rn(__fmul_rn(wmu, p.delZk), w.yx), sig, gd, w.ay, ws, we, dr, di);
+    else hat_diag(w.zy, sx, w.zx, sy, __fmul_rn(__fmul_rn(wmu, p.dzk), w.az), sig, gd, w.az, ws, we, dr, di);
 }
 
-// y / D and |D|^2 (the fast reciprocal intrinsic: D^-1 only has to be the
-// same in every kernel that applies it, which one function guarantees)
-__device__ __forceinline__ float2 hat_div(float2 y, float dr, float di, float &W)
+// y / D and |D|^2, both zero unless `in` (the approximate reciprocal: D^-1 only
+// has to be the same in every kernel that applies it, which one function
+// guarantees)
+__device__ __forceinline__ float2 hat_div(float2 y, float dr, float di, bool in, float &W)
 {
-    W = dr * dr + di * di;
-    const float inv = __fdividef(1.f, W);
+    W = __fmaf_rn(dr, dr, __fmul_rn(di, di));
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(W));
+    inv = in ? inv : 0.f;
+    W = in ? W : 0.f;
     return make_float2((y.x * dr + y.y * di) * inv, (y.y * dr - y.x * di) * inv);
 }
 
@@ -119,8 +137,8 @@ __global__ void __launch_bounds__(kThreads) kh_cast(KArgs<float> a, const double
                 wne = a.gdn[q.c == 0 ? ns + 1 : q.c == 1 ? ns + g.nx + 1 : ns + (g.nx + 1) * (g.ny + 1)];
             }
             float dr, di, W;
-            hat_diag(q.c, cg, pg, wmu, a.sigma[e], a.gd != 0, wns, wne, dr, di);
-            rh = hat_div(b, dr, di, W);
+            hat_diag_of(q.c, cg, pg, hat_coef(cg, pg), wmu, a.sigma[e], a.gd != 0, wns, wne, dr, di);
+            rh = hat_div(b, dr, di, true, W);
             y = make_float2(dr * b.x + di * b.y, dr * b.y - di * b.x);  // conj(D) b
             u[0] += (double)b.x * b.x + (double)b.y * b.y;
         }
@@ -266,44 +284,109 @@ __device__ __forceinline__ void hat_xr(const KArgs<float> &a, int r, int bx)
 // divided by D at the edge
 // ---------------------------------------------------------------------------
 
+// an entry read once, left out of the L1 cache (28 KB beside the ring), where the
+// plane tables stay
+__device__ __forceinline__ float2 load_once(const float2 *p)
+{
+    float2 v;
+    asm volatile("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+
+// grad-div potential of a node, |w| sum of C_e DFA_e x_e over its edges (k_gd_phi
+// mode 0), from the fields before and after it along each axis; S and Sz are at
+// its sigma in the planes of the node and below it.  Nodes on the boundary have
+// the weight zero, and so the potential
+__device__ __forceinline__ float2 hat_phi(float wn, float2 xm, float2 x, float2 ym, float2 y, float2 zm, float2 z,
+                                          const float *S, const float *Sz, float dX, float dY, float dZ)
+{
+    constexpr int SW = HatTile::SW, cs = HatTile::FR * SW;
+    const bool earth = wn < 0.f;  // C = sigma_E, or one at air nodes
+    const auto c = [&](float sig) { return earth ? sig : 1.f; };
+    const float2 u = csub(cscale(xm, c(S[-1])), cscale(x, c(S[0])));
+    const float2 v = csub(cscale(ym, c(S[cs - SW])), cscale(y, c(S[cs])));
+    const float2 w = csub(cscale(zm, c(Sz[2 * cs])), cscale(z, c(S[2 * cs])));
+    return cscale(cadd(cadd(cscale(u, dY * dZ), cscale(v, dX * dZ)), cscale(w, dX * dY)), fabsf(wn));
+}
+// a (after - before) - b (after - before) of two pairs: a curl's component
+__device__ __forceinline__ float2 hat_curl(float2 p1, float2 p0, float a, float2 q1, float2 q0, float b)
+{
+    return csub(cscale(csub(p1, p0), a), cscale(csub(q1, q0), b));
+}
+
 // March planes [k0, k1) of tile (i0, j0), right-hand side r, calling
 // f(e, yhat, x_e, W, aux_e) for the three edge slots (Ex, Ey, Ez) of every
 // node of the thread's two columns, padding slots included: yhat =
 // D^-1 (A x)_e and W = |D_e|^2 at interior edges (zero otherwise), e the
 // padded index, aux_e the entry of the vector aux (read one plane ahead,
-// zero when aux is null).  A block of kHatThreads threads covers the 16 x 16
-// node tile: thread (tx, ty) takes the node columns (i0 + tx, j0 + ty) and
-// (i0 + tx, j0 + ty + 8), so the per-plane work of a thread (waits,
-// barriers, plane geometry, loop control) is shared by six edges and the
-// register budget of four blocks per SM is 128 per thread.  Returns false
-// (all threads of the block alike) when a wait gave up.
+// zero when aux is null).  A thread (tx, ty) of the 128 takes the node columns
+// (i0 + tx, j0 + 2 ty) and (i0 + tx, j0 + 2 ty + 1), so the per-plane work of a thread
+// (waits, barriers, plane geometry, loop control) is shared by six edges, the
+// columns share their row's fields, and the register budget of four blocks per
+// SM is 128 per thread.  Returns false (all threads of the block alike) when a
+// wait gave up.
+//
+// curl curl is taken in two steps, as it is defined: the curl on the faces
+// after a node,
+//   Hx = dEz/dy - dEy/dz,  Hy = dEx/dz - dEz/dx,  Hz = dEy/dx - dEx/dy,
+// once for the four edges around each face, then the curl of that on the
+// edges times V_E.  The faces below a node come from its own previous plane,
+// those before it along x from the lane before (or the tile's halo column),
+// along y from the thread's own pair or from the row published in shared
+// memory.  The kernel is bound by instruction issue.  With every edge forming its
+// eight differences anew (60 complex operations a node for the curls, here 24;
+// 30 reads of staged fields, here 21 for two nodes), the diagonal's products
+// formed edge by edge and the potentials behind tests, a launch took on average
+// over the four of an iteration, in us: 40^3, 8 right-hand sides 25.6, now 23.6;
+// 64 x 64 x 48, 8: 61, now 53.3; 100 x 100 x 60, 2: 43.6, now 36.6; 200 x 200 x
+// 100, 1: 111, now 93; 4: 376, now 312.  Of that the plane tables in registers
+// give 2 % (they fell out of the L1 cache, 28 KB beside the ring, and were
+// waited for on every plane), and the pairs of rows four apart 2 to 3 %.
 template <bool gd, typename F>
 __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp, const Geo<float> &g, PadLayout pl, int r,
                                           const float2 *__restrict__ aux, float wmu, int i0, int j0, int k0, int k1,
                                           int *err, int limit, F &&f)
 {
-    const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
-    const int i = i0 + tx, jA = j0 + ty, jB = jA + kHatRows;
+    const int tx = threadIdx.x % kTX, warp = threadIdx.x >> 5;
+    const bool side = (threadIdx.x & 16) != 0;
+    // the pair of rows: a warp's two are four rows apart, 80 words of sigma or
+    // node weights, so that its halves read different banks
+    const int ty = (warp & 1) + 4 * (warp >> 1) + (side ? 2 : 0);
+    const int i = i0 + tx, jA = j0 + 2 * ty, jB = jA + 1;
     const bool liveA = i <= g.nx && jA <= g.ny, liveB = i <= g.nx && jB <= g.ny;
     const ColGeo<float> cgA = col_geo(g, min(i, g.nx), min(jA, g.ny));
     const ColGeo<float> cgB = col_geo(g, min(i, g.nx), min(jB, g.ny));
-    const int hfA = (ty + 1) * kFW + tx + 2;  // own column in a field plane of the tile
-    const int hsA = (ty + 1) * kSW + tx + 1;  // own column in a sigma plane
-    const int hnA = ty * kPhX + tx;           // own node in a potential plane
-    const int hwA = ty * kNW + tx;            // own node in a node-weight plane
-    constexpr int dF = kHatRows * kFW, dS = kHatRows * kSW, dN = kHatRows * kPhX, dW = kHatRows * kNW;
-    const int cf = kFR * kFW, cs = kFR * kSW;
+    // of the first column; the second is one row on
+    const int hf = (2 * ty + 1) * kFW + tx + 2;  // in a field plane of the tile
+    const int hs = (2 * ty + 1) * kSW + tx + 1;  // in a sigma plane
+    const int hn = 2 * ty * kPhX + tx;           // in a potential plane
+    const int hw = 2 * ty * kNW + tx;            // in a node-weight plane
+    constexpr int cf = kFR * kFW, cs = kFR * kSW;
     const int pxy = pl.Px * pl.Py, pc = pl.Pz * pxy;
     const int colA = min(i, pl.Px - 1) + pl.Px * min(jA, pl.Py - 1);
     const int colB = min(i, pl.Px - 1) + pl.Px * min(jB, pl.Py - 1);
     const bool issuer = threadIdx.x == 0;
     const unsigned tx_bytes = kFBytes + kSBytes;
-    // halo nodes of the potentials: (i0 + 32, j0 .. j0 + 8) and (i0 .. i0 + 31, j0 + 8)
-    const bool hasH = threadIdx.x < kTX + kTY + 1;
-    const int hni = threadIdx.x < kTX ? threadIdx.x : kTX;
-    const int hnj = threadIdx.x < kTX ? kTY : threadIdx.x - kTX;
+    // the halo, half a warp a side.  Warp 0: potentials of the nodes (i0 .. i0 +
+    // 15, j0 + 16) and (i0 + 16, j0 .. j0 + 15).  Warp 2: curls of the row j0 - 1
+    // and of the column i0 - 1
+    const int hni = side ? kTX : tx, hnj = side ? tx : kTY;
     const int hi = i0 + hni, hj = j0 + hnj;
-    const float hdX = (hasH && hi <= g.nx) ? g.delX[hi] : 0.f, hdY = (hasH && hj <= g.ny) ? g.delY[hj] : 0.f;
+    float hdX = 0.f, hdY = 0.f;       // warp 0: the node's widths
+    float hrN = 0.f, hrT = 0.f;       // warp 2: 1 / d across the row or column and along it
+    if (gd && warp == 0) {
+        hdX = hi <= g.nx ? g.delX[hi] : 0.f;
+        hdY = hj <= g.ny ? g.delY[hj] : 0.f;
+    }
+    if (warp == 2) {
+        if (!side) {
+            hrN = j0 >= 1 ? g.rdy[j0 - 1] : 0.f;
+            hrT = i < g.nx ? g.rdx[i] : 0.f;
+        } else {
+            hrN = i0 >= 1 ? g.rdx[i0 - 1] : 0.f;
+            hrT = j0 + tx < g.ny ? g.rdy[j0 + tx] : 0.f;
+        }
+    }
 
     // a chunk past the last node plane (the last chunks when the chunk count
     // does not divide the planes) has no work; it must return before it
@@ -314,25 +397,26 @@ __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp
         return false;
     }
     if (issuer) {
-        for (int q = 0; q < 4; q++) mbar_init(smem_addr(&sm.mbar[q]), 1);
+        for (int q = 0; q < HatTile::Ring; q++) mbar_init(smem_addr(&sm.mbar[q]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     __syncthreads();
     unsigned phase = 0;
+    const auto slot_of = [&](int p) { return (p - k0 + 1) % HatTile::Ring; };  // p >= k0 - 1
+    const auto after = [](int s) { return s == HatTile::Ring - 1 ? 0 : s + 1; };
     // node weights are staged for planes k0 .. k1 (the diagonal and the
     // potentials need them), in slot p & 1
     auto issue = [&](int p) {
         if (!issuer) return;
-        const int s = p & 3;
+        const int s = slot_of(p);
         const bool node = gd && p >= k0;
         const unsigned mb = smem_addr(&sm.mbar[s]);
         mbar_expect(mb, tx_bytes + (node ? kNBytes : 0u));
         tma_load4(smem_addr(sm.fld[s]), &tp.in, 2 * (i0 - 2), j0 - 1, p, 3 * r, mb);
-        tma_load4(smem_addr(sm.sig[mod3(p)]), &tp.sig, i0, j0 - 1, p, 0, mb);
+        tma_load4(smem_addr(sm.sig[p & 3]), &tp.sig, i0, j0 - 1, p, 0, mb);
         if (node) tma_load3(smem_addr(sm.nod[p & 1]), &tp.node, i0, j0, p, mb);
     };
-    auto wait = [&](int p) -> bool {
-        const int s = p & 3;
+    auto wait = [&](int s) -> bool {
         if (mbar_wait(smem_addr(&sm.mbar[s]), (phase >> s) & 1u, limit)) {
             phase ^= 1u << s;
             return true;
@@ -342,28 +426,48 @@ __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp
     auto give_up = [&](int first, int last) {
         if (!issuer) return;
         atomicExch(err, 1);
-        for (int q = first; q <= last; q++)
-            if (mbar_wait(smem_addr(&sm.mbar[q & 3]), (phase >> (q & 3)) & 1u, kWaitLimit)) phase ^= 1u << (q & 3);
-    };
-    auto phi_plane = [&](int p) {
-        const float dZ = (p >= 0 && p <= g.nz) ? g.delZ[p] : 0.f;
-        float2 *P = sm.phi[p & 1];
-        P[hnA] = tma_phi_node<HatTile>(sm, g, i, jA, p, tx, ty, cgA.delXi, cgA.delYj, dZ);
-        P[hnA + dN] = tma_phi_node<HatTile>(sm, g, i, jB, p, tx, ty + kHatRows, cgB.delXi, cgB.delYj, dZ);
-        if (hasH) P[hnj * kPhX + hni] = tma_phi_node<HatTile>(sm, g, hi, hj, p, hni, hnj, hdX, hdY, dZ);
+        for (int q = first; q <= last; q++) {
+            const int s = slot_of(q);
+            if (mbar_wait(smem_addr(&sm.mbar[s]), (phase >> s) & 1u, kWaitLimit)) phase ^= 1u << s;
+        }
     };
     const float2 zero = make_float2(0.f, 0.f);
-    // signed node weights of each column's nodes (i, j), (i+1, j), (i, j+1)
-    // at the plane being computed
-    float wSA = 0.f, wXA = 0.f, wYA = 0.f, wSB = 0.f, wXB = 0.f, wYB = 0.f;
-    auto node_w = [&](int p, float &sa, float &xa, float &ya, float &sb, float &xb, float &yb) {
+    const auto field = [&](int s) { return reinterpret_cast<const float2 *>(sm.fld[s]); };
+    const auto sigma = [&](int p) { return reinterpret_cast<const float *>(sm.sig[p & 3]); };
+    // potentials of the thread's nodes at plane p (fields in slot s, those
+    // below in slot sb), and of a halo node
+    struct Phi {
+        float2 a, b, halo;
+    };
+    auto phi_form = [&](int p, int s, int sb, float dZ) {
+        Phi v = {zero, zero, zero};
+        const float2 *X = field(s), *Y = X + cf, *Z = Y + cf, *Zb = field(sb) + 2 * cf;
+        const float *S = sigma(p), *Sb = sigma(p - 1), *N = reinterpret_cast<const float *>(sm.nod[p & 1]);
+        const auto at = [&](int h, int q, float wn, float dX, float dY) {
+            return hat_phi(wn, X[h - 1], X[h], Y[h - kFW], Y[h], Zb[h], Z[h], S + q, Sb + q, dX, dY, dZ);
+        };
+        v.a = at(hf, hs, N[hw], cgA.delXi, cgA.delYj);
+        v.b = at(hf + kFW, hs + kSW, N[hw + kNW], cgB.delXi, cgB.delYj);
+        if (warp == 0)
+            v.halo = at((hnj + 1) * kFW + hni + 2, (hnj + 1) * kSW + hni + 1, N[hnj * kNW + hni], hdX, hdY);
+        return v;
+    };
+    auto phi_put = [&](int p, const Phi &v) {
+        float2 *P = sm.phi[p & 1];
+        P[hn] = v.a;
+        P[hn + kPhX] = v.b;
+        if (warp == 0) P[hnj * kPhX + hni] = v.halo;
+    };
+    // signed node weights of the columns' nodes at the plane being computed:
+    // (i, j), (i, j + 1), (i, j + 2), (i + 1, j), (i + 1, j + 1)
+    float w0[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    auto node_w = [&](int p, float (&w)[5]) {
         const float *N = reinterpret_cast<const float *>(sm.nod[p & 1]);
-        sa = N[hwA];
-        xa = N[hwA + 1];
-        ya = N[hwA + kNW];
-        sb = N[hwA + dW];
-        xb = N[hwA + dW + 1];
-        yb = N[hwA + dW + kNW];
+        w[0] = N[hw];
+        w[1] = N[hw + kNW];
+        w[2] = N[hw + 2 * kNW];
+        w[3] = N[hw + 1];
+        w[4] = N[hw + kNW + 1];
     };
     // (padding entries of aux, where Ex, Ey or Ez does not exist, are zero)
     float2 axA = zero, ayA = zero, azA = zero, axB = zero, ayB = zero, azB = zero;
@@ -371,151 +475,174 @@ __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp
         if (!aux || k > g.nz) return;
         if (liveA) {
             const int b = colA + pxy * k;
-            axA = aux[b];
-            ayA = aux[pc + b];
-            azA = aux[2 * pc + b];
+            axA = load_once(aux + b);
+            ayA = load_once(aux + pc + b);
+            azA = load_once(aux + 2 * pc + b);
         }
         if (liveB) {
             const int b = colB + pxy * k;
-            axB = aux[b];
-            ayB = aux[pc + b];
-            azB = aux[2 * pc + b];
+            axB = load_once(aux + b);
+            ayB = load_once(aux + pc + b);
+            azB = load_once(aux + 2 * pc + b);
         }
     };
 
-    // the three edges of one node column at plane k.  Every edge slot is
-    // formed without branches: an edge that is not interior (or does not
-    // exist: Ex at i = nx, Ey at j = ny, Ez at k = nz, all padding entries
-    // of the layout) gets yhat = 0 and W = 0, so it adds nothing to the
-    // inner products and keeps its zero.  The shared-memory reads stay
+    // the three edges of one node column at plane k from the fields x, y, z on
+    // them and the curls around them: H*, before it along x (i), y (j) and z
+    // (k).  Every edge slot is formed without branches: an edge that is not
+    // interior (or does not exist: Ex at i = nx, Ey at j = ny, Ez at k = nz, all
+    // padding entries of the layout) gets yhat = 0 and W = 0, so it adds nothing
+    // to the inner products and keeps its zero.  The shared-memory reads stay
     // inside the tile whatever the edge.
-    auto node_edges = [&](const ColGeo<float> &cg, const PlaneGeo<float> &pg, int k, bool kin, int h, int hs, int hn,
-                          float wS, float wX, float wY, float nS, int eb, float2 ax, float2 ay, float2 az) {
-        const float2 *Fm = reinterpret_cast<const float2 *>(sm.fld[(k - 1) & 3]);
-        const float2 *F0 = reinterpret_cast<const float2 *>(sm.fld[k & 3]);
-        const float2 *Fp = reinterpret_cast<const float2 *>(sm.fld[(k + 1) & 3]);
-        const float *S0 = reinterpret_cast<const float *>(sm.sig[k % 3]);
-        const float2 *Xm = Fm, *X0 = F0, *Xp = Fp;
-        const float2 *Ym = Fm + cf, *Y0 = F0 + cf, *Yp = Fp + cf;
-        const float2 *Zm = Fm + 2 * cf, *Z0 = F0 + 2 * cf;
-        const float2 *P0 = sm.phi[k & 1], *P1 = sm.phi[(k + 1) & 1];
-        // ---- Ex(i, j, k)
-        {
-            const float2 X1 = X0[h];
-            const bool in = cg.intX && kin;
+    auto node_edges = [&](const ColGeo<float> &cg, const PlaneGeo<float> &pg, int k, int q, int n, float wS, float wX,
+                          float wY, float wZ, float2 p1, int eb, float2 x, float2 y, float2 z, float2 Hx, float2 Hxj, float2 Hxk,
+                          float2 Hy, float2 Hyi, float2 Hyk, float2 Hz, float2 Hzi, float2 Hzj, float2 ax, float2 ay,
+                          float2 az) {
+        const float *S0 = sigma(k) + q;
+        const float2 *P0 = sm.phi[k & 1] + n;
+        const bool kin = k >= 1 && k <= g.nz - 1;
+        const float2 p0 = gd ? P0[0] : zero;
+        // A x from its real part, then i omega mu0 sigma V_E x and D^-1
+        const HatCoef w = hat_coef(cg, pg);
+        const auto edge = [&](int comp, bool in, int e, float2 out, float2 v, float sig, float w1, float2 a) {
             float dr, di, W;
-            hat_diag(0, cg, pg, wmu, S0[hs], gd, wS, wX, dr, di);
-            const float2 yy = csub(cadd(csub(Y0[h + 1], Y0[h]), Y0[h - kFW]), Y0[h + 1 - kFW]);
-            const float2 zz = csub(cadd(csub(Z0[h + 1], Z0[h]), Zm[h]), Zm[h + 1]);
-            const float2 fyp = cscale(csub(X0[h + kFW], X1), cg.rdyj);
-            const float2 fym = cscale(csub(X1, X0[h - kFW]), cg.rdyjm1);
-            const float2 fzp = cscale(csub(Xp[h], X1), pg.rdzk);
-            const float2 fzm = cscale(csub(X1, Xm[h]), pg.rdzkm1);
-            float2 out = cadd(cscale(yy, pg.delZk), cscale(zz, cg.delYj));
-            out = csub(out, cscale(csub(fyp, fym), cg.dxi * pg.delZk));
-            out = csub(out, cscale(csub(fzp, fzm), cg.dxi * cg.delYj));
-            out.x -= di * X1.y;
-            out.y += di * X1.x;
-            if (gd) out = cadd(out, cscale(csub(P0[hn + 1], P0[hn]), cg.delYj * pg.delZk));
-            out = hat_div(out, dr, di, W);
-            f(eb, in ? out : zero, X1, in ? W : 0.f, ax);
+            hat_diag_of(comp, cg, pg, w, wmu, sig, gd, wS, w1, dr, di);
+            out.x -= di * v.y;
+            out.y += di * v.x;
+            out = hat_div(out, dr, di, in, W);
+            f(e, out, v, W, a);
+        };
+        {
+            float2 out = csub(cscale(csub(Hz, Hzj), w.xz), cscale(csub(Hy, Hyk), w.xy));
+            if (gd) out = cadd(out, cscale(csub(P0[1], p0), w.ax));
+            edge(0, cg.intX && kin, eb, out, x, S0[0], wX, ax);
         }
-        // ---- Ey(i, j, k)
         {
-            const float2 Y1 = Y0[h];
-            const bool in = cg.intY && kin;
-            float dr, di, W;
-            hat_diag(1, cg, pg, wmu, S0[cs + hs], gd, wS, wY, dr, di);
-            const float2 zz = csub(cadd(csub(Z0[h + kFW], Z0[h]), Zm[h]), Zm[h + kFW]);
-            const float2 xx = csub(cadd(csub(X0[h + kFW], X0[h]), X0[h - 1]), X0[h - 1 + kFW]);
-            const float2 fzp = cscale(csub(Yp[h], Y1), pg.rdzk);
-            const float2 fzm = cscale(csub(Y1, Ym[h]), pg.rdzkm1);
-            const float2 fxp = cscale(csub(Y0[h + 1], Y1), cg.rdxi);
-            const float2 fxm = cscale(csub(Y1, Y0[h - 1]), cg.rdxim1);
-            float2 out = cadd(cscale(zz, cg.delXi), cscale(xx, pg.delZk));
-            out = csub(out, cscale(csub(fzp, fzm), cg.dyj * cg.delXi));
-            out = csub(out, cscale(csub(fxp, fxm), cg.dyj * pg.delZk));
-            out.x -= di * Y1.y;
-            out.y += di * Y1.x;
-            if (gd) out = cadd(out, cscale(csub(P0[hn + kPhX], P0[hn]), cg.delXi * pg.delZk));
-            out = hat_div(out, dr, di, W);
-            f(pc + eb, in ? out : zero, Y1, in ? W : 0.f, ay);
+            float2 out = csub(cscale(csub(Hx, Hxk), w.yx), cscale(csub(Hz, Hzi), w.yz));
+            if (gd) out = cadd(out, cscale(csub(P0[kPhX], p0), w.ay));
+            edge(1, cg.intY && kin, pc + eb, out, y, S0[cs], wY, ay);
         }
-        // ---- Ez(i, j, k)
         {
-            const float2 Z1 = Z0[h];
-            const bool in = cg.intZ && k < g.nz;
-            float dr, di, W;
-            hat_diag(2, cg, pg, wmu, S0[2 * cs + hs], gd, wS, nS, dr, di);
-            const float2 xx = csub(cadd(csub(Xp[h], X0[h]), X0[h - 1]), Xp[h - 1]);
-            const float2 yy = csub(cadd(csub(Yp[h], Y0[h]), Y0[h - kFW]), Yp[h - kFW]);
-            const float2 fxp = cscale(csub(Z0[h + 1], Z1), cg.rdxi);
-            const float2 fxm = cscale(csub(Z1, Z0[h - 1]), cg.rdxim1);
-            const float2 fyp = cscale(csub(Z0[h + kFW], Z1), cg.rdyj);
-            const float2 fym = cscale(csub(Z1, Z0[h - kFW]), cg.rdyjm1);
-            float2 out = cadd(cscale(xx, cg.delYj), cscale(yy, cg.delXi));
-            out = csub(out, cscale(csub(fxp, fxm), pg.dzk * cg.delYj));
-            out = csub(out, cscale(csub(fyp, fym), pg.dzk * cg.delXi));
-            out.x -= di * Z1.y;
-            out.y += di * Z1.x;
-            if (gd) out = cadd(out, cscale(csub(P1[hn], P0[hn]), cg.delXi * cg.delYj));
-            out = hat_div(out, dr, di, W);
-            f(2 * pc + eb, in ? out : zero, Z1, in ? W : 0.f, az);
+            float2 out = csub(cscale(csub(Hy, Hyi), w.zy), cscale(csub(Hx, Hxj), w.zx));
+            if (gd) out = cadd(out, cscale(csub(p1, p0), w.az));
+            edge(2, cg.intZ && k < g.nz, 2 * pc + eb, out, z, S0[2 * cs], wZ, az);
         }
     };
+    const auto lane_before = [](float2 v) {
+        return make_float2(__shfl_up_sync(0xffffffffu, v.x, 1, kTX), __shfl_up_sync(0xffffffffu, v.y, 1, kTX));
+    };
 
+    // the plane tables, 32 planes from kt on, a plane a lane
+    int kt = 0;
+    float tdz = 0.f, tdelZ = 0.f, trdz = 0.f, rdzk = k0 > 0 ? g.rdz[k0 - 1] : 0.f;
+    auto tables = [&](int k) {
+        kt = k;
+        const int q = k + (threadIdx.x & 31);
+        tdz = q < g.nz ? g.dz[q] : 0.f;
+        trdz = q < g.nz ? g.rdz[q] : 0.f;
+        tdelZ = g.delZ[min(q, g.nz)];
+    };
+    tables(k0);
     load_aux(k0);
     issue(k0 - 1);
     issue(k0);
     issue(k0 + 1);
+    int s0 = 0, s1 = 1;  // slots of the plane marched and the one after it
+    float2 HxAk = zero, HyAk = zero, HxBk = zero, HyBk = zero;  // curls of the plane before
     {
-        const bool w0 = wait(k0 - 1), w1 = w0 && wait(k0);
-        if (w1 && gd) {
-            phi_plane(k0);
-            node_w(k0, wSA, wXA, wYA, wSB, wXB, wYB);
-        }
-        if (!__syncthreads_and(w1)) {
-            give_up(w1 ? k0 + 1 : w0 ? k0 : k0 - 1, k0 + 1);
-            return false;
-        }
-    }
-    // One barrier per plane.  Plane k reads the potentials of plane k at the
-    // thread's node and at its +x and +y neighbours, published by the
-    // barrier that ended the previous plane, and those of plane k + 1 at its
-    // own node only, which it has just formed; so it can be computed as soon
-    // as the thread's own wait for plane k + 1 has completed.  The barrier at
-    // the end publishes plane k + 1's potentials, frees the ring slots of
-    // plane k - 1 for the copies the next plane issues, and makes a wait
-    // that gave up end the block as a whole.
-    for (int k = k0; k < k1; k++) {
-        const int last = k + 2 <= k1 ? k + 2 : k + 1;
-        if (k + 2 <= k1) issue(k + 2);
-        const bool ok = wait(k + 1);
-        float nSA = 0.f, nXA = 0.f, nYA = 0.f, nSB = 0.f, nXB = 0.f, nYB = 0.f;  // plane k + 1
-        if (ok) {
+        const bool r0 = wait(s0), r1 = r0 && wait(s1);
+        if (r1) {
+            const float rdz = rdzk;
+            const float2 *X0 = field(s0) + hf, *Y0 = X0 + cf, *Z0 = Y0 + cf, *X1 = field(s1) + hf, *Y1 = X1 + cf;
+            HyAk = hat_curl(X1[0], X0[0], rdz, Z0[1], Z0[0], cgA.rdxi);
+            HyBk = hat_curl(X1[kFW], X0[kFW], rdz, Z0[kFW + 1], Z0[kFW], cgB.rdxi);
+            HxAk = hat_curl(Z0[kFW], Z0[0], cgA.rdyj, Y1[0], Y0[0], rdz);
+            HxBk = hat_curl(Z0[2 * kFW], Z0[kFW], cgB.rdyj, Y1[kFW], Y0[kFW], rdz);
             if (gd) {
-                phi_plane(k + 1);
-                node_w(k + 1, nSA, nXA, nYA, nSB, nXB, nYB);
+                phi_put(k0, phi_form(k0, s1, s0, g.delZ[k0]));
+                node_w(k0, w0);
             }
-            const PlaneGeo<float> pg = plane_geo(g, k);
-            const bool kin = k >= 1 && k <= g.nz - 1;
-            if (liveA)
-                node_edges(cgA, pg, k, kin, hfA, hsA, hnA, wSA, wXA, wYA, nSA, colA + pxy * k, axA, ayA, azA);
-            if (liveB)
-                node_edges(cgB, pg, k, kin, hfA + dF, hsA + dS, hnA + dN, wSB, wXB, wYB, nSB, colB + pxy * k, axB,
-                           ayB, azB);
-            if (k + 1 < k1) load_aux(k + 1);
         }
-        wSA = nSA;
-        wXA = nXA;
-        wYA = nYA;
-        wSB = nSB;
-        wXB = nXB;
-        wYB = nYB;
-        if (!__syncthreads_and(ok)) {
-            give_up(ok ? k + 2 : k + 1, last);
+        if (!__syncthreads_and(r1)) {
+            give_up(r1 ? k0 + 1 : r0 ? k0 : k0 - 1, k0 + 1);
             return false;
         }
+        if (k0 + 2 <= k1) issue(k0 + 2);
+        s0 = s1;
+        s1 = after(s1);
+    }
+    // One barrier per plane.  Before it the thread forms the curls of plane k
+    // and the potentials of plane k + 1, as soon as its own wait for plane k +
+    // 1 has completed, and keeps the fields and sigma of its edges; the
+    // barrier publishes the curls, frees the field slot of plane k for the copy
+    // issued after it, and makes a wait that gave up end the block as a whole.
+    // After it come the edges of plane k, and the potentials of plane k + 1 take
+    // the place of plane k - 1's, which no thread reads any more; what the
+    // edges of plane k read is written again past the next barrier at the
+    // earliest.
+    for (int k = k0; k < k1; k++) {
+        const bool ok = wait(s1);
+        if (k + 1 >= kt + 32) tables(k);
+        const float dZ1 = __shfl_sync(0xffffffffu, tdelZ, k + 1 - kt);
+        const PlaneGeo<float> pg = {__shfl_sync(0xffffffffu, tdz, k - kt), __shfl_sync(0xffffffffu, tdelZ, k - kt),
+                                    __shfl_sync(0xffffffffu, trdz, k - kt), rdzk};
+        rdzk = pg.rdzk;
+        // (what a wait that gave up leaves here is not used)
+        const float2 *X0 = field(s0) + hf, *Y0 = X0 + cf, *Z0 = Y0 + cf, *X1 = field(s1) + hf, *Y1 = X1 + cf;
+        const float2 xA = X0[0], yA = Y0[0], zA = Z0[0], xB = X0[kFW], yB = Y0[kFW], zB = Z0[kFW];
+        const float2 HxA = hat_curl(zB, zA, cgA.rdyj, Y1[0], yA, pg.rdzk);
+        const float2 HyA = hat_curl(X1[0], xA, pg.rdzk, Z0[1], zA, cgA.rdxi);
+        const float2 HzA = hat_curl(Y0[1], yA, cgA.rdxi, xB, xA, cgA.rdyj);
+        const float2 HxB = hat_curl(Z0[2 * kFW], zB, cgB.rdyj, Y1[kFW], yB, pg.rdzk);
+        const float2 HyB = hat_curl(X1[kFW], xB, pg.rdzk, Z0[kFW + 1], zB, cgB.rdxi);
+        const float2 HzB = hat_curl(Y0[kFW + 1], yB, cgB.rdxi, X0[2 * kFW], xB, cgB.rdyj);
+        if (warp == 2) {
+            // T along the row or column, N across it
+            const int h = side ? (tx + 1) * kFW + 1 : tx + 2, sN = side ? 1 : kFW, sT = side ? kFW : 1;
+            const float2 *T0 = field(s0) + h + (side ? 0 : cf), *T1 = field(s1) + h + (side ? 0 : cf);
+            const float2 *N0 = field(s0) + h + (side ? cf : 0), *Zh = field(s0) + h + 2 * cf;
+            const float2 a = hat_curl(Zh[sN], Zh[0], hrN, T1[0], T0[0], pg.rdzk);
+            const float2 b = hat_curl(T0[sT], T0[0], hrT, N0[sN], N0[0], hrN);
+            if (side) {
+                sm.lefty[k & 1][tx] = make_float2(-a.x, -a.y);
+                sm.leftz[k & 1][tx] = make_float2(-b.x, -b.y);
+            } else {
+                sm.hx[k & 1][0][tx] = a;
+                sm.hz[k & 1][0][tx] = b;
+            }
+        }
+        sm.hx[k & 1][ty + 1][tx] = HxB;
+        sm.hz[k & 1][ty + 1][tx] = HzB;
+        float w1[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // plane k + 1
+        Phi p1 = {zero, zero, zero};
+        if (gd) {
+            p1 = phi_form(k + 1, s1, s0, dZ1);
+            node_w(k + 1, w1);
+        }
+        if (!__syncthreads_and(ok)) {
+            give_up(ok ? k + 2 : k + 1, min(k + 2, k1));
+            return false;
+        }
+        if (k + 3 <= k1) issue(k + 3);
+        if (gd) phi_put(k + 1, p1);
+        float2 HyAi = lane_before(HyA), HzAi = lane_before(HzA), HyBi = lane_before(HyB), HzBi = lane_before(HzB);
+        if (tx == 0) {
+            HyAi = sm.lefty[k & 1][2 * ty];
+            HzAi = sm.leftz[k & 1][2 * ty];
+            HyBi = sm.lefty[k & 1][2 * ty + 1];
+            HzBi = sm.leftz[k & 1][2 * ty + 1];
+        }
+        if (liveA)
+            node_edges(cgA, pg, k, hs, hn, w0[0], w0[3], w0[1], w1[0], p1.a, colA + pxy * k, xA, yA, zA, HxA, sm.hx[k & 1][ty][tx],
+                       HxAk, HyA, HyAi, HyAk, HzA, HzAi, sm.hz[k & 1][ty][tx], axA, ayA, azA);
+        if (liveB)
+            node_edges(cgB, pg, k, hs + kSW, hn + kPhX, w0[1], w0[4], w0[2], w1[1], p1.b, colB + pxy * k, xB, yB, zB, HxB, HxA,
+                       HxBk, HyB, HyBi, HyBk, HzB, HzBi, HzA, axB, ayB, azB);
+        if (k + 1 < k1) load_aux(k + 1);
+        HxAk = HxA, HyAk = HyA, HxBk = HxB, HyBk = HyB;
+        for (int q = 0; q < 5; q++) w0[q] = w1[q];
+        s0 = s1;
+        s1 = after(s1);
     }
     return true;
 }

@@ -1088,10 +1088,10 @@ int Solver::solve_begin(SolveRun &run, int nrhs, const double *omegas, const int
 // recursion goes on falling where FP32 can no longer lower the true residual
 // (some 1e-6 of the cycle's start), so a cycle that reaches this has nothing
 // left to gain and the next one goes on from the true residual.  Solves to 1e-12
-// on 19 grids of 24^3 to 200 x 200 x 100 cells took 6 % less time with 3e-7 (24^3:
-// 12.8 -> 9.4 ms), 5 % with 1e-7, 6 to 7 % with 1e-6 to 1e-5; solves to 1e-7 the
-// same to 1 % with all of them.
-constexpr double kInnerFloor = 3e-7;
+// on 19 grids of 24^3 to 200 x 200 x 100 cells took 5 % less time with 1e-7, 6 to 7 %
+// with 3e-7 to 1e-5; but those split a solve to 1e-7, the default tolerance, into
+// one more cycle.
+constexpr double kInnerFloor = 1e-7;
 
 // start of an outer cycle: the true FP64 residual r64 = b - A X (into tmp);
 // converged right-hand sides leave the loop; the FP32 and FP64 groups of the

@@ -62,15 +62,31 @@ template <int TX_, int TY_> struct TmaTile {
 // the unfused kernels (tmakernels.cu): a thread per node column
 using KctTile = TmaTile<32, 8>;
 static_assert(KctTile::TX * KctTile::TY == kThreads, "one thread per node column");
-// the fused stencil (hatkernels.cu): 128 threads, each on two node rows (ty and
-// ty + 8).  A row of 16 wastes at most 15 lanes on a grid's rim where one of 32
+// the fused stencil (hatkernels.cu): 128 threads, each on two node rows next to
+// one another.  A row of 16 wastes at most 15 lanes on a grid's rim where one of 32
 // wastes up to 31 (65 nodes take 80 columns instead of 96, 41 take 48 instead
 // of 64, 201 take 208 instead of 224), at the same halo a tile.  us a launch
 // against a 32 x 8 tile: 40^3, 8 right-hand sides 25.6 (30.5); 100 x 100 x 60, 2:
 // 44.3 (47.5); 200 x 200 x 100, 4: 380 (392).
-using HatTile = TmaTile<16, 16>;
-constexpr int kHatThreads = 128, kHatRows = HatTile::TY / 2;
-static_assert(kHatThreads == HatTile::TX * kHatRows, "fused stencil thread layout");
+// Its ring holds the fields of three planes (k and k + 1 in use until the curls
+// of plane k are formed, then k + 1, k + 2 and k + 3), sigma of four and the
+// node weights of two; the curls that cross threads or tiles (hx, hz: the row
+// before each thread's pair; left: the column before the tile) and the
+// potentials are kept for two planes, so that one barrier a plane is enough.
+constexpr int kHatThreads = 128, kHatPairs = 8;
+struct HatTile : TmaTile<16, 16> {
+    static constexpr int Ring = 3;
+    struct Smem {
+        alignas(128) unsigned char fld[Ring][slot(FBytes)];
+        alignas(128) unsigned char sig[4][slot(SBytes)];
+        alignas(128) unsigned char nod[2][slot(NBytes)];
+        float2 phi[2][PhN];
+        float2 hx[2][kHatPairs + 1][TX], hz[2][kHatPairs + 1][TX];
+        float2 lefty[2][TY], leftz[2][TY];
+        unsigned long long mbar[Ring];
+    };
+};
+static_assert(kHatThreads == HatTile::TX * kHatPairs && 2 * kHatPairs == HatTile::TY, "fused stencil thread layout");
 static_assert(4 * (sizeof(HatTile::Smem) + 1024) <= 228 * 1024, "four blocks of the fused stencil on an SM");
 __device__ __forceinline__ int mod3(int p) { return ((p % 3) + 3) % 3; }
 

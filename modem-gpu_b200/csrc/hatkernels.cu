@@ -37,11 +37,11 @@
 // the solve.)
 //
 // The operator kernels stage u or sh with the tensor copies of tma.cuh.  D =
-// V_E xXO-diagonal of the curl-curl term (col_ccdiag) + the grad-div diagonal
+// V_E xXO-diagonal of the curl-curl term + the grad-div diagonal
 // DFA^2 (w_s c_s + w_e c_e) + i omega mu0 sigma V_E, from the staged sigma
-// and signed node weights (the weights of each node column's three nodes at
-// plane k are kept in registers from the previous plane, so the node ring
-// keeps two slots).  kh_cast computes the same D from the global tables.
+// and signed node weights (those of a plane are kept in registers from the
+// plane before, so the node ring keeps two slots).  kh_cast computes the same D
+// from the global tables.
 #include <atomic>
 #include <cstring>
 
@@ -319,7 +319,7 @@ __device__ __forceinline__ float2 hat_curl(float2 p1, float2 p0, float a, float2
 // node of the thread's two columns, padding slots included: yhat =
 // D^-1 (A x)_e and W = |D_e|^2 at interior edges (zero otherwise), e the
 // padded index, aux_e the entry of the vector aux (read one plane ahead,
-// zero when aux is null).  A thread (tx, ty) of the 128 takes the node columns
+// zero without has_aux).  A thread (tx, ty) of the 128 takes the node columns
 // (i0 + tx, j0 + 2 ty) and (i0 + tx, j0 + 2 ty + 1), so the per-plane work of a thread
 // (waits, barriers, plane geometry, loop control) is shared by six edges, the
 // columns share their row's fields, and the register budget of four blocks per
@@ -337,12 +337,12 @@ __device__ __forceinline__ float2 hat_curl(float2 p1, float2 p0, float a, float2
 // eight differences anew (60 complex operations a node for the curls, here 24;
 // 30 reads of staged fields, here 21 for two nodes), the diagonal's products
 // formed edge by edge and the potentials behind tests, a launch took on average
-// over the four of an iteration, in us: 40^3, 8 right-hand sides 25.6, now 23.6;
-// 64 x 64 x 48, 8: 61, now 53.3; 100 x 100 x 60, 2: 43.6, now 36.6; 200 x 200 x
-// 100, 1: 111, now 93; 4: 376, now 312.  Of that the plane tables in registers
+// over the four of an iteration, in us: 40^3, 8 right-hand sides 25.6, now 23.1;
+// 64 x 64 x 48, 8: 61, now 52.5; 100 x 100 x 60, 2: 43.6, now 36.4; 200 x 200 x
+// 100, 1: 111, now 92; 4: 376, now 308.  Of that the plane tables in registers
 // give 2 % (they fell out of the L1 cache, 28 KB beside the ring, and were
 // waited for on every plane), and the pairs of rows four apart 2 to 3 %.
-template <bool gd, typename F>
+template <bool gd, bool has_aux, typename F>
 __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp, const Geo<float> &g, PadLayout pl, int r,
                                           const float2 *__restrict__ aux, float wmu, int i0, int j0, int k0, int k1,
                                           int *err, int limit, F &&f)
@@ -469,22 +469,18 @@ __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp
         w[3] = N[hw + 1];
         w[4] = N[hw + kNW + 1];
     };
-    // (padding entries of aux, where Ex, Ey or Ez does not exist, are zero)
+    // (padding entries of aux, where Ex, Ey or Ez does not exist, are zero; the
+    // columns are clamped into the layout, so every lane loads)
     float2 axA = zero, ayA = zero, azA = zero, axB = zero, ayB = zero, azB = zero;
     auto load_aux = [&](int k) {
-        if (!aux || k > g.nz) return;
-        if (liveA) {
-            const int b = colA + pxy * k;
-            axA = load_once(aux + b);
-            ayA = load_once(aux + pc + b);
-            azA = load_once(aux + 2 * pc + b);
-        }
-        if (liveB) {
-            const int b = colB + pxy * k;
-            axB = load_once(aux + b);
-            ayB = load_once(aux + pc + b);
-            azB = load_once(aux + 2 * pc + b);
-        }
+        if (!has_aux) return;
+        const float2 *p = aux + pxy * k;
+        axA = load_once(p + colA);
+        ayA = load_once(p + colA + pc);
+        azA = load_once(p + colA + 2 * pc);
+        axB = load_once(p + colB);
+        ayB = load_once(p + colB + pc);
+        azB = load_once(p + colB + 2 * pc);
     };
 
     // the three edges of one node column at plane k from the fields x, y, z on
@@ -681,16 +677,14 @@ __device__ __forceinline__ void hat_vt(const TmaParams &tp, const KArgs<float> &
     // after a restart (first iteration, pad set) the shadow becomes the
     // current residual: y = W rh, rh being the staged u of this launch
     const bool reset = (stage == 0 || stage == 2) && st.first && st.pad;
-    const float2 *aux = nullptr;
-    if (kv && !reset) aux = Yr;
-    if (stage == 5) aux = a.sh + off;
+    const float2 *aux = kv ? Yr : stage == 5 ? a.sh + off : nullptr;
     const float c2 = 2.f * a.pc, cc = a.pc * a.pc;
     // inner products summed per edge in FP64 (per-plane FP32 partial sums
     // changed the Krylov rounding enough to send more right-hand sides to
     // the FP64 fallback)
     double u[4] = {0.0, 0.0, 0.0, 0.0};
     HatTile::Smem &sm = tma_smem<HatTile>();
-    const bool ok = hat_march<gd>(
+    const bool ok = hat_march<gd, kv || stage == 5>(
         sm, tp, a.g, a.pl, r, aux, (float)(a.dsgn * a.ost[r].omega * kMu0), i0, j0, k0, k1, a.err, a.wait_limit,
         // y and W are zero at edges that are not interior, and so are x
         // and xa there (u, sh, w1, w2 and the shadow vanish off the

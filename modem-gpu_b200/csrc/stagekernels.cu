@@ -171,7 +171,7 @@ template <typename K> static int stage_setup(K kern, size_t smem, int slot)
 // Time of a launch of c chunks of len planes (the last of them shorter) over
 // `layer` blocks each, in planes of a block that has its SM to itself.  A block
 // costs a plane and a half to start; each further block on an SM slows all of
-// them down by a fifth (the fused FP32 stencil: 1.55, 1.85, 2.2 and 2.5 us a
+// them down by a fifth (the fused FP32 stencil when fitted: 1.55, 1.85, 2.2 and 2.5 us a
 // plane with one to four blocks, so latency counts for more than throughput).
 // Full waves come first; the blocks of the last chunk fill the slots that the
 // others leave, as work that can be shared out, and a quarter of one at the end.
@@ -189,8 +189,8 @@ static double stage_time(long layer, int c, int len, int last, long resident)
 // GPU that holds `resident` blocks.  The blocks of right-hand sides that have
 // converged exit at once, so half and one of them running count a quarter each
 // beside all running.  Against the best of all counts measured over 24^3 to
-// 200 x 200 x 100 cells and 1 to 8 right-hand sides the choice takes 1.3 % more
-// time for the fused FP32 stencil and 1.0 % for the FP64 one (mean; 7 % at
+// 200 x 200 x 100 cells and 1 to 8 right-hand sides the choice takes 1.9 % more
+// time for the fused FP32 stencil and 1.0 % for the FP64 one (mean; 12 and 7 % at
 // most), and 8 % with half of them left; one count for a single right-hand side
 // in chunks of at least 8 planes took 22.3 instead of 10.9 us a launch on 24^3
 // cells with 2 right-hand sides.

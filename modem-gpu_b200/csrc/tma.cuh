@@ -66,8 +66,9 @@ static_assert(KctTile::TX * KctTile::TY == kThreads, "one thread per node column
 // one another.  A row of 16 wastes at most 15 lanes on a grid's rim where one of 32
 // wastes up to 31 (65 nodes take 80 columns instead of 96, 41 take 48 instead
 // of 64, 201 take 208 instead of 224), at the same halo a tile.  us a launch
-// against a 32 x 8 tile: 40^3, 8 right-hand sides 25.6 (30.5); 100 x 100 x 60, 2:
-// 44.3 (47.5); 200 x 200 x 100, 4: 380 (392).
+// against a 32 x 8 tile, both with every edge forming its own differences: 40^3,
+// 8 right-hand sides 25.6 (30.5); 100 x 100 x 60, 2: 44.3 (47.5); 200 x 200 x 100,
+// 4: 380 (392).
 // Its ring holds the fields of three planes (k and k + 1 in use until the curls
 // of plane k are formed, then k + 1, k + 2 and k + 3), sigma of four and the
 // node weights of two; the curls that cross threads or tiles (hx, hz: the row

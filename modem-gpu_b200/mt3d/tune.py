@@ -1,8 +1,9 @@
 """Launch-shape tuning of multi-grid batches (mt3d_fwdsolve_multi).
 
-The FP32 stencil kernels give each block a tile of 32 x 8 node columns and a
-chunk of the node planes; how many chunks a grid's columns are split into
-trades the blocks' start-up (three planes staged before the first is
+The FP32 stencil kernels give each block a tile of node columns (16 x 16 the
+fused ones, 32 x 8 the unfused) and a chunk of the node planes; how many
+chunks a grid's columns are split into trades the blocks' start-up (three
+planes staged before the first is
 computed) against filling the GPU's resident slots in few, full waves.  The
 library picks the count from an occupancy model of one grid alone; in a
 multi-grid batch the grids share every launch, so the best split of each

@@ -171,8 +171,9 @@ template <typename K> static int stage_setup(K kern, size_t smem, int slot)
 // Time of a launch of c chunks of len planes (the last of them shorter) over
 // `layer` blocks each, in planes of a block that has its SM to itself.  A block
 // costs a plane and a half to start; each further block on an SM slows all of
-// them down by a fifth (the fused FP32 stencil when fitted: 1.55, 1.85, 2.2 and 2.5 us a
-// plane with one to four blocks, so latency counts for more than throughput).
+// them down by a fifth (the fused FP32 stencil when fitted: 1.55, 1.85, 2.2 and
+// 2.5 us a plane with one to four blocks, so latency counts for more than
+// throughput).
 // Full waves come first; the blocks of the last chunk fill the slots that the
 // others leave, as work that can be shared out, and a quarter of one at the end.
 static double stage_time(long layer, int c, int len, int last, long resident)

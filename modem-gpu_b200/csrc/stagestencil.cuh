@@ -223,7 +223,12 @@ __device__ __forceinline__ void stage_march(StageSmem<T> &sm, const Geo<T> &g, c
     stage_plane(sm, g, map, x, sig, gdn, k0 + 1);
     cp_async_wait_all();
     __syncthreads();
-    if (gd) phi_plane(k0);
+    if (gd) {
+        phi_plane(k0);
+        // plane k0 + 2's node weights go into the slot of plane k0, which the
+        // potentials of every warp have to have read
+        __syncthreads();
+    }
     for (int k = k0; k < k1; k++) {
         stage_plane(sm, g, map, x, sig, gdn, k + 2);
         if (gd) phi_plane(k + 1);

@@ -559,6 +559,7 @@ __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp
                 node_w(k0, w0);
             }
         }
+        slots_read();
         if (!__syncthreads_and(r1)) {
             give_up(r1 ? k0 + 1 : r0 ? k0 : k0 - 1, k0 + 1);
             return false;
@@ -615,6 +616,7 @@ __device__ __forceinline__ bool hat_march(HatTile::Smem &sm, const TmaParams &tp
             p1 = phi_form(k + 1, s1, s0, dZ1);
             node_w(k + 1, w1);
         }
+        slots_read();
         if (!__syncthreads_and(ok)) {
             give_up(ok ? k + 2 : k + 1, min(k + 2, k1));
             return false;

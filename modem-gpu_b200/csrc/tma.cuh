@@ -134,6 +134,13 @@ __device__ __forceinline__ void tma_load3(unsigned dst, const CUtensorMap *m, in
         : "memory");
 }
 
+// Before a barrier after which a copy may go into a slot: the thread's reads of
+// the slot are done.  Tensor copies write through the async proxy, which a
+// barrier alone does not order after the reads of other threads through the
+// generic one, so a value read before the barrier and used after it may be
+// fetched late, from the plane that took its place.
+__device__ __forceinline__ void slots_read() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+
 // grad-div potential of node (ni, nj) of the tile (global i, j) at plane p:
 // the sums of k_gd_phi (mode 0) in the same order, from the staged planes
 template <typename Tile>

@@ -137,6 +137,7 @@ __device__ __forceinline__ bool tma_march(KctTile::Smem &sm, const TmaParams &tp
         if (w1 && gd) phi_plane(k0);
         // plane k0 + 2 goes into the sigma slot of plane k0 - 1 and the node
         // slot of plane k0, which the potentials of plane k0 have just read
+        slots_read();
         if (!__syncthreads_and(w1)) {
             give_up(w1 ? k0 + 1 : w0 ? k0 : k0 - 1, k0 + 1);
             return false;
@@ -232,6 +233,7 @@ __device__ __forceinline__ bool tma_march(KctTile::Smem &sm, const TmaParams &tp
             }
             if (k + 1 < k1) load_aux(k + 1);
         }
+        slots_read();
         __syncthreads();
     }
     return true;

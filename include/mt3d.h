@@ -307,6 +307,13 @@ MT3D_API int mt3d_set_stream(mt3d_handle h, void *stream);
  * fault. */
 MT3D_API int mt3d_set_wait_limit(mt3d_handle h, int polls);
 
+/* Chunks of node planes that the staged stencil kernels split a grid into (no
+ * counterpart in the reference); 0, the default, lets every launch choose.
+ * Counts above the nz + 1 planes mean one chunk a plane.  The results change by
+ * the order of sums only: for timing a split, and for checking the kernels with
+ * chunks of every length. */
+MT3D_API int mt3d_set_chunks(mt3d_handle h, int chunks);
+
 /* y = A x on FULL edge vectors in host memory through one of the library's
  * internal operator kernels, for checking the kernels against each other and
  * against an independent operator (no counterpart in the reference; the

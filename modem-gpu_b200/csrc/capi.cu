@@ -346,6 +346,11 @@ int mt3d_set_wait_limit(mt3d_handle h, int polls)
     return wrap(h, [&] { return h->s.set_wait_limit(polls); });
 }
 
+int mt3d_set_chunks(mt3d_handle h, int chunks)
+{
+    return wrap(h, [&] { return h->s.set_chunks(chunks); });
+}
+
 int mt3d_apply_kernel(mt3d_handle h, int kernel, const double *x, double *y)
 {
     return wrap(h, [&] { return h->s.apply_kernel(kernel, x, y); });

@@ -811,8 +811,8 @@ template <int stage, bool gd> static void launch_hat_vt_t(const KArgs<float> &a,
 {
     const size_t sm = sizeof(HatTile::Smem);
     const int res = tma_resident(kh_vt<stage, gd>, sm, 2 + 2 * stage + (gd ? 1 : 0), kHatThreads);
-    kh_vt<stage, gd><<<dim3(a.hmap.tiles, nrhs, stage_chunks(a.g.nz, a.hmap.tiles, res, nrhs)), kHatThreads, sm, s>>>(
-        tp, a);
+    const int zc = a.zchunks ? a.zchunks : stage_chunks(a.g.nz, a.hmap.tiles, res, nrhs);
+    kh_vt<stage, gd><<<dim3(a.hmap.tiles, nrhs, zc), kHatThreads, sm, s>>>(tp, a);
 }
 template <int stage> static void launch_hat_stage(const KArgs<float> &a, int nrhs, cudaStream_t s)
 {
@@ -1066,7 +1066,8 @@ int launch_hat_iter_multi(const KArgs<float> *args, const int *nrhs, const int *
         // time is flat about it: 262 to 273 ms for 40^3 + 64 x 64 x 48 cells with
         // counts from 3, 5 to 11, 13); more chunks than planes would only add
         // empty ones, and the reductions' partial sums have room for one a plane
-        p.zch[g] = std::min(zch && zch[g] > 0 ? zch[g] : stage_chunks(args[g].g.nz, args[g].hmap.tiles, res, nrhs[g]),
+        const int own = args[g].zchunks;
+        p.zch[g] = std::min(zch && zch[g] > 0 ? zch[g] : own ? own : stage_chunks(args[g].g.nz, args[g].hmap.tiles, res, nrhs[g]),
                             args[g].g.nz + 1);
         p.eb0[g + 1] = p.eb0[g] + nrhs[g] * args[g].nblk;
         p.sb0[g + 1] = p.sb0[g] + nrhs[g] * args[g].hmap.tiles * p.zch[g];

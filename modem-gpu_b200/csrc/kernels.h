@@ -99,6 +99,7 @@ template <typename T> struct KArgs {
     PadLayout pl;
     int *err;        // set by a bounded device-side wait that gave up
     int wait_limit;  // polls of one bounded wait before it gives up
+    int zchunks;     // chunks of node planes of the staged stencils; 0: the launch's own choice (stage_chunks)
     const struct TmaMaps *tma;  // host pointer: tensor maps of the padded vectors (colstencil == 3)
     // profiling: the staged stencil kernels count one sweep per active
     // right-hand side and launch here (nullptr when not profiling)

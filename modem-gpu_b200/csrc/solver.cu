@@ -68,6 +68,13 @@ int Solver::set_wait_limit(int polls)
     return 0;
 }
 
+int Solver::set_chunks(int chunks)
+{
+    if (chunks < 0) return fail(5, "mt3d_set_chunks: the count must not be negative");
+    zchunks_ = std::min(chunks, nz + 1);
+    return 0;
+}
+
 int Solver::profile(int enable)
 {
     if (stream_) cudaStreamSynchronize(stream_);
@@ -481,6 +488,7 @@ template <> KArgs<double> Solver::kargs<double>(int nrhs, int)
     a.nblk = blocks_for(nE, a.chunk);
     a.len = (int)nE;
     a.err = errf_.as<int>();
+    a.zchunks = zchunks_;
     a.maxit = ctl.IterPerDivCor;
     a.inner = 0;
     a.dsgn = -1.0;
@@ -526,6 +534,7 @@ template <> KArgs<float> Solver::kargs<float>(int nrhs, int)
     a.len = (int)nE;
     a.err = errf_.as<int>();
     a.wait_limit = wait_limit_;
+    a.zchunks = zchunks_;
     a.pc = (float)ctl.poly;
     if (w.padded) {
         // padded layout: the elementwise kernels sweep the padded length and

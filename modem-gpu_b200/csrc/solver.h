@@ -132,6 +132,7 @@ class Solver {
     int device() const { return dev_; }
     int set_stream(void *s);
     int set_wait_limit(int polls);
+    int set_chunks(int chunks);
     int set_fused(int on);
     int set_poly(double c);
     int profile(int enable);
@@ -206,6 +207,7 @@ class Solver {
     DevBuf sigP32_, sigsP32_, gdnP32_, errf_;
     TmaMaps *tma_ = nullptr;
     int wait_limit_ = 1 << 22;  // polls of a bounded device-side wait
+    int zchunks_ = 0;           // caller's plane chunks of the staged stencils (0: the library's)
     bool tma_stale_ = true;
     int tma_ready();
     int check_device_error(const char *what);

@@ -223,7 +223,9 @@ template <typename T> static dim3 stage_grid(const KArgs<T> &a, int nrhs, int re
     // per cent from the true one: there the sums keep the order of the count for
     // one right-hand side in chunks of at least 8 planes
     int c = 1;
-    if (a.gd) {
+    if (a.zchunks) {
+        c = a.zchunks;
+    } else if (a.gd) {
         c = stage_chunks(a.g.nz, a.cmap.tiles, resident, nrhs);
     } else {
         const int planes = a.g.nz + 1;

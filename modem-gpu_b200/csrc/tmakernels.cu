@@ -382,7 +382,7 @@ void launch_tma_init(const KArgs<float> &a, const TmaMaps *m, int nrhs, cudaStre
     tp.node = m->node;
     const size_t sm = sizeof(KctTile::Smem);
     const int res = tma_resident(kct_init, sm, 0);
-    kct_init<<<dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kThreads, sm, s>>>(tp, a);
+    kct_init<<<dim3(a.cmap.tiles, nrhs, a.zchunks ? a.zchunks : stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kThreads, sm, s>>>(tp, a);
 }
 void launch_tma_vt(const KArgs<float> &a, const TmaMaps *m, int which, int nrhs, cudaStream_t s)
 {
@@ -393,7 +393,7 @@ void launch_tma_vt(const KArgs<float> &a, const TmaMaps *m, int which, int nrhs,
     tp.node = m->node;
     const size_t sm = sizeof(KctTile::Smem);
     const int res = tma_resident(kct_vt, sm, 1);
-    kct_vt<<<dim3(a.cmap.tiles, nrhs, stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kThreads, sm, s>>>(tp, a, which);
+    kct_vt<<<dim3(a.cmap.tiles, nrhs, a.zchunks ? a.zchunks : stage_chunks(a.g.nz, a.cmap.tiles, res, nrhs)), kThreads, sm, s>>>(tp, a, which);
 }
 
 }  // namespace mt3d

@@ -27,7 +27,7 @@ EXPORTS = ["mt3d_version", "mt3d_device_count", "mt3d_create", "mt3d_destroy", "
            "mt3d_get_cond", "mt3d_compute_bc", "mt3d_compute_bc_device", "mt3d_update_freq", "mt3d_set_formulation", "mt3d_set_restart", "mt3d_sizes", "mt3d_interior_index", "mt3d_mult_aii",
            "mt3d_mult_aii_device_noalloc", "mt3d_bicg", "mt3d_fwdsolve",
            "mt3d_fwdsolve_batch", "mt3d_fwdsolve_batch_device", "mt3d_fwdsolve_multi",
-           "mt3d_fwdsolve_multi_device", "mt3d_set_stream", "mt3d_set_wait_limit", "mt3d_set_fused",
+           "mt3d_fwdsolve_multi_device", "mt3d_set_stream", "mt3d_set_wait_limit", "mt3d_set_chunks", "mt3d_set_fused",
            "mt3d_set_poly",
            "mt3d_apply_kernel", "mt3d_profile",
            "mt3d_kernel_time", "mt3d_get_diag", "mt3d_get_batch_diag", "mt3d_pmult_t", "mt3d_impedance", "mt3d_impedance_device", "mt3d_lmult_t", "mt3d_lmult_t_device", "mt3d_jmult_t", "mt3d_jmult_t_device", "mt3d_write_soln", "mt3d_read_soln", "mt3d_read_soln_header", "mt3d_launch_counter", "mt3d_alloc_counter",
@@ -95,6 +95,7 @@ def load(path: str = LIB_PATH):
     L.mt3d_fwdsolve_batch_device.argtypes = [P, I, D, IP, C.c_void_p, C.c_void_p, C.c_void_p, IP]
     L.mt3d_set_stream.argtypes = [P, C.c_void_p]
     L.mt3d_set_wait_limit.argtypes = [P, I]
+    L.mt3d_set_chunks.argtypes = [P, I]
     PP = C.POINTER(C.c_void_p)
     for name in ("mt3d_fwdsolve_multi", "mt3d_fwdsolve_multi_device"):
         getattr(L, name).argtypes = [I, C.POINTER(P), IP, PP, PP, PP, PP, PP, PP, IP]
@@ -383,6 +384,10 @@ class Solver:
 
     def set_wait_limit(self, polls: int):
         self._check(self.L.mt3d_set_wait_limit(self.h, int(polls)))
+
+    def set_chunks(self, chunks: int):
+        """Chunks of node planes of the staged stencils (0: the library's choice)."""
+        self._check(self.L.mt3d_set_chunks(self.h, int(chunks)))
 
     def apply_kernel(self, kernel: int, x: np.ndarray) -> np.ndarray:
         """A x on full edge vectors through internal kernel 0 (FP64 apply),

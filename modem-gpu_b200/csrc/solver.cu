@@ -1093,14 +1093,19 @@ int Solver::solve_begin(SolveRun &run, int nrhs, const double *omegas, const int
     return 0;
 }
 
-// How far an FP32 cycle takes its own residual at most.  The iteration's
-// recursion goes on falling where FP32 can no longer lower the true residual
-// (some 1e-6 of the cycle's start), so a cycle that reaches this has nothing
-// left to gain and the next one goes on from the true residual.  Solves to 1e-12
-// on 19 grids of 24^3 to 200 x 200 x 100 cells took 5 % less time with 1e-7, 6 to 7 %
-// with 3e-7 to 1e-5; but those split a solve to 1e-7, the default tolerance, into
-// one more cycle.
-constexpr double kInnerFloor = 1e-7;
+// How far an FP32 cycle takes its own residual while cycles are left.  The
+// iteration's recursion goes on falling below what FP32 leaves of the true
+// residual (3e-7 to 1e-4 of the cycle's start on grids of 24^3 to 64 x 64 x 48
+// cells), so below 1e-7 little is gained and the next cycle goes on from the true
+// residual.  Solves of 15 pairs of right-hand sides (24^3 to 100 x 100 x 60 cells,
+// 0.1 to 10 Hz), geometric means in ms, without and with: to 1e-12 47.5, 44.0; to
+// 1e-10 39.0, 36.0; to 1e-9 33.8, 32.4; to 1e-8 28.6, 28.4; to 1e-7 24.8, 24.9.
+// A cycle that ends there leaves up to 1e-7 more than one that runs on, which a call
+// of few cycles cannot make good (with two of them and 1e-10, 40^3 cells stopped at
+// 1.04e-10 instead of 0.94e-10).  So it ends there only if the cycles after it reach the
+// tolerance at a thousandth each, and runs to the tolerance otherwise: at up to
+// three cycles the calls of 136 settings end exactly as without.
+constexpr double kInnerFloor = 1e-7, kCycleGain = 1e-3;
 
 // start of an outer cycle: the true FP64 residual r64 = b - A X (into tmp);
 // converged right-hand sides leave the loop; the FP32 and FP64 groups of the
@@ -1132,7 +1137,9 @@ int Solver::solve_pre(SolveRun &run)
             if (!std::isfinite(o.relres)) { o.active = 0; o.failed = 3; continue; }
             if (o.relres <= o.tol) { o.active = 0; o.converged = 1; continue; }
             if (o.nDivCor >= ctl.MaxDivCor) { o.active = 0; o.failed = 1; continue; }
-            o.tol_inner = std::max(o.tol * o.bnorm64 * o.scale, kInnerFloor);  // tol*||b|| relative to ||r64||
+            o.tol_inner = o.tol * o.bnorm64 * o.scale;  // tol*||b|| relative to ||r64||
+            if (o.tol_inner < kInnerFloor && std::pow(kCycleGain, ctl.MaxDivCor - o.nDivCor - 1) <= o.tol_inner)
+                o.tol_inner = kInnerFloor;
             // an FP32 cycle that did not halve the true residual: when its
             // own iteration converged well, the FP32 operator's rounding is
             // the limit and the right-hand side moves to FP64; when the

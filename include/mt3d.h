@@ -327,6 +327,12 @@ MT3D_API int mt3d_set_chunks(mt3d_handle h, int chunks);
  *             (mt3d_set_fused): y = D^-1 A x, D = diag(A), x rounded to FP32. */
 MT3D_API int mt3d_apply_kernel(mt3d_handle h, int kernel, const double *x, double *y);
 
+/* The reciprocals that the 2-D boundary solver divides by (mt3d_compute_bc), for
+ * checking them against a division (no counterpart in the reference): for n
+ * complex numbers z in host memory y[i] = 1 / Re z[i] and w[i] = 1 / z[i]
+ * (complex).  y is defined where Re z and 1 / Re z are normal numbers. */
+MT3D_API int mt3d_check_reciprocal(mt3d_handle h, int n, const double *z, double *y, double *w);
+
 /* Kernel timing: with enable != 0 every launch of the BiCGStab stencil
  * kernels (v = A ph with the fused dot product) is bracketed by CUDA events
  * on the solver stream.  mt3d_kernel_time returns, for the launches of one

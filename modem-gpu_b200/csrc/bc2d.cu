@@ -60,15 +60,32 @@ __device__ __forceinline__ double2 cdv(double2 a, double2 b)
     return c2((a.x * r + a.y) / den, (a.y * r - a.x) / den);
 }
 
-// 1 / x for normal x: the hardware's approximation y (2^-23 or better, so e =
-// 1 - x y is small) and the first terms of 1 / x = y (1 + e + e^2 + ...), three
-// dependent operations; what is dropped, e^3, lies below the last bit
+// 1 / x for x and 1 / x normal: one step of the hyperpower iteration of order
+// three (M. Altman, Pacific J. Math. 10, 1960), y (1 + e + e^2) with e = 1 - x y,
+// from the approximate reciprocal y of the PTX instruction.  That reads the upper
+// 32 bits of x, 20 of them mantissa, and returns 20 bits of mantissa (PTX ISA,
+// rcp.approx.ftz.f64): |e| <= 2^-19.  What is dropped, e^3, is at most 2^-57, an
+// eighth of the last bit's half; with the last rounding the result is within one
+// unit in the last place of the rounded 1 / x.  Three dependent operations after
+// the instruction, where a division has some ten.
 __device__ __forceinline__ double rcp_fast(double x)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
+}
+// 1 / z for any z: conj(z) / |z|^2 where |z|^2 is far from over- and underflow,
+// as with all but absurd frequencies and cell sizes, Smith's algorithm otherwise
+// (out of line: inlined five times in a panel's sweep it made 40^3 cells 5 % slower;
+// the test itself costs 0 to 2.5 %)
+__device__ __noinline__ double2 crcp_far(double2 z) { return cdv(c2(1.0, 0.0), z); }
+__device__ __forceinline__ double2 crcp(double2 z)
+{
+    const double n = fma(z.x, z.x, z.y * z.y);
+    if (!(n > 1e-290 && n < 1e290)) return crcp_far(z);
+    const double iv = rcp_fast(n);
+    return c2(z.x * iv, -z.y * iv);
 }
 
 struct Slice {
@@ -118,9 +135,7 @@ __global__ void k_bc1d(BcArgs a)
     double2 *xs = side >= 0 ? a.side + ((size_t)s * 2 + side) * (nz + 1) : nullptr;
     // row j: ad_{j-1} x_{j-1} + ac_j x_j + ad_j x_{j+1} = r_j, r_0 = -au_0
     // the conductivities and widths of kAhead rows are read ahead of the chain,
-    // whose step is one complex reciprocal (the entries are of the size of
-    // inverse layer thicknesses and of omega mu sigma times a thickness: their
-    // squares neither overflow nor vanish): 40 us for the columns of 40^3
+    // whose step is one complex reciprocal: 40 us for the columns of 40^3
     // cells, 107 us for 200 x 200 x 100, against 56 and 172 us with the loads
     // and six divisions a row on the chain
     constexpr int kAhead = 8;
@@ -141,8 +156,7 @@ __global__ void k_bc1d(BcArgs a)
             if (j >= nz) break;
             const double ad = an[q], ss = sn[q] * dn[q] + sk * dk;
             const double2 den = c2(-au - ad - adprev * cprev.x, a.omue * ss - adprev * cprev.y);
-            const double iv = rcp_fast(fma(den.x, den.x, den.y * den.y));
-            const double2 id = c2(den.x * iv, -den.y * iv);
+            const double2 id = crcp(den);
             const double2 r = c2((j == 0 ? -au : 0.0) - adprev * dprev.x, -adprev * dprev.y);
             cprev = c2(ad * id.x, ad * id.y);
             dprev = cm(r, id);
@@ -295,8 +309,8 @@ __global__ void k_bc_coef(BcArgs a, int nslices)
 // Bound by FP64 arithmetic for long lines (half of m^3 complex multiply-adds
 // a line) and by the panels' chains for short ones.  One polarisation, against
 // the band elimination of k_bc2d (a pivot at a time, two block barriers and
-// the whole window through shared memory for each): 200 x 200 x 100 cells 18.2
-// against 208.4 ms, 101 x 83 x 61 1.68 against 17.8 ms, 40^3 0.37 against
+// the whole window through shared memory for each): 200 x 200 x 100 cells 18.7
+// against 208.4 ms, 101 x 83 x 61 1.69 against 17.8 ms, 40^3 0.38 against
 // 4.66 ms.  (8 x 8 blocks in FP64 matrix instructions, which run at the same
 // rate, were slower: 20.6 to 27.9 ms for the first.)  The error against dense 64-bit solves is the same (2e-14).
 // ---------------------------------------------------------------------------
@@ -441,10 +455,7 @@ template <bool mid, int threads, int blocks> __global__ void __launch_bounds__(t
                 double2 l[T];
 #pragma unroll
                 for (int r = 0; r < T; r++) l[r] = shfl2(v[r], kBcOwn + p);
-                // the pivots are of the size of ratios of cell widths and of omega
-                // mu sigma times a cell's area: their squares neither overflow nor vanish
-                const double den = rcp_fast(fma(l[p].x, l[p].x, l[p].y * l[p].y));
-                const double2 iv = c2(l[p].x * den, -l[p].y * den);
+                const double2 iv = crcp(l[p]);
                 const bool pc = col == P + p;
                 const double2 g = pc ? iv : cm(v[p], iv);
 #pragma unroll
@@ -951,6 +962,31 @@ int launch_bc2d(const BcArgs &a, int nblocks, bool window_in_smem, cudaStream_t 
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
     k_bc2d<<<nblocks, block, smem, s>>>(a, window_in_smem ? 1 : 0);
     return (int)cudaGetLastError();
+}
+
+// the elimination's reciprocals as they stand: y = 1 / Re z, w = 1 / z
+__global__ void __launch_bounds__(256) k_bc_reciprocal(int n, const double2 *z, double *y, double2 *w)
+{
+    const int t = blockIdx.x * 256 + threadIdx.x;
+    if (t >= n) return;
+    y[t] = rcp_fast(z[t].x);
+    w[t] = crcp(z[t]);
+}
+
+int Solver::check_reciprocal(int n, const double *z, double *y, double *w)
+{
+    const char *who = "mt3d_check_reciprocal";
+    if (n < 1 || !z || !y || !w) return fail(5, std::string(who) + ": invalid arguments");
+    const size_t b = (size_t)n * sizeof(double);
+    DevBuf dz, dy, dw;
+    if (dz.alloc(2 * b) || dy.alloc(b) || dw.alloc(2 * b)) return fail(8, std::string(who) + ": out of device memory");
+    cudaMemcpyAsync(dz.as<void>(), z, 2 * b, cudaMemcpyHostToDevice, stream_);
+    g_launch_count.fetch_add(1, std::memory_order_relaxed);
+    k_bc_reciprocal<<<(unsigned)(((long long)n + 255) / 256), 256, 0, stream_>>>(n, dz.as<double2>(), dy.as<double>(),
+                                                                                 dw.as<double2>());
+    cudaMemcpyAsync(y, dy.as<void>(), b, cudaMemcpyDeviceToHost, stream_);
+    cudaMemcpyAsync(w, dw.as<void>(), 2 * b, cudaMemcpyDeviceToHost, stream_);
+    return sync(who);
 }
 
 // ---------------------------------------------------------------------------

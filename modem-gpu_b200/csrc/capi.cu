@@ -356,6 +356,11 @@ int mt3d_apply_kernel(mt3d_handle h, int kernel, const double *x, double *y)
     return wrap(h, [&] { return h->s.apply_kernel(kernel, x, y); });
 }
 
+int mt3d_check_reciprocal(mt3d_handle h, int n, const double *z, double *y, double *w)
+{
+    return wrap(h, [&] { return h->s.check_reciprocal(n, z, y, w); });
+}
+
 int mt3d_profile(mt3d_handle h, int enable)
 {
     return wrap(h, [&] { return h->s.profile(enable); });

@@ -108,6 +108,7 @@ class Solver {
     int mult_aii(int adjt, const double *x, double *y);
     int mult_aii_noalloc(int adjt, const double *x, double *y);  // device vectors, fixed scratch
     int apply_kernel(int kernel, const double *x, double *y);   // one internal operator kernel
+    int check_reciprocal(int n, const double *z, double *y, double *w);
     int bicg(const double *b, double *x, int maxit, double tol, int *niter, double *rerr, int *failed);
     int solve(int nrhs, const double *omegas, const int *trans, const double *bc, const double *src, double *e,
               int *status, bool device = false);

@@ -29,7 +29,7 @@ EXPORTS = ["mt3d_version", "mt3d_device_count", "mt3d_create", "mt3d_destroy", "
            "mt3d_fwdsolve_batch", "mt3d_fwdsolve_batch_device", "mt3d_fwdsolve_multi",
            "mt3d_fwdsolve_multi_device", "mt3d_set_stream", "mt3d_set_wait_limit", "mt3d_set_chunks", "mt3d_set_fused",
            "mt3d_set_poly",
-           "mt3d_apply_kernel", "mt3d_profile",
+           "mt3d_apply_kernel", "mt3d_check_reciprocal", "mt3d_profile",
            "mt3d_kernel_time", "mt3d_get_diag", "mt3d_get_batch_diag", "mt3d_pmult_t", "mt3d_impedance", "mt3d_impedance_device", "mt3d_lmult_t", "mt3d_lmult_t_device", "mt3d_jmult_t", "mt3d_jmult_t_device", "mt3d_write_soln", "mt3d_read_soln", "mt3d_read_soln_header", "mt3d_launch_counter", "mt3d_alloc_counter",
            "mt3d_last_error"]
 
@@ -104,6 +104,7 @@ def load(path: str = LIB_PATH):
     L.mt3d_jmult_t.argtypes = [P, C.c_double, I, D, D, D, D, D, D, D]
     L.mt3d_jmult_t_device.argtypes = [P, C.c_double, I, D, D, C.c_void_p, D, D, C.c_void_p, C.c_void_p]
     L.mt3d_apply_kernel.argtypes = [P, I, D, D]
+    L.mt3d_check_reciprocal.argtypes = [P, I, D, D, D]
     L.mt3d_profile.argtypes = [P, I]
     L.mt3d_kernel_time.argtypes = [P, I, IP, D, C.POINTER(C.c_int64)]
     L.mt3d_get_diag.argtypes = [P, IP, IP, IP, D, I, D, I, D]
@@ -397,6 +398,13 @@ class Solver:
         y = np.zeros(self.nE, np.complex128)
         self._check(self.L.mt3d_apply_kernel(self.h, int(kernel), _d(x), _d(y)))
         return y
+
+    def check_reciprocal(self, z):
+        """(1 / z.real, 1 / z) as the boundary solver forms them."""
+        z = np.ascontiguousarray(z, dtype=np.complex128)
+        y, w = np.zeros(z.size), np.zeros(z.size, np.complex128)
+        self._check(self.L.mt3d_check_reciprocal(self.h, z.size, _d(z), _d(y), _d(w)))
+        return y, w
 
     def profile(self, enable=True):
         self._check(self.L.mt3d_profile(self.h, int(enable)))

@@ -55,7 +55,14 @@ constexpr int kTX = HatTile::TX, kTY = HatTile::TY, kFW = HatTile::FW, kFR = Hat
 constexpr unsigned kFBytes = HatTile::FBytes, kSBytes = HatTile::SBytes, kNBytes = HatTile::NBytes;
 
 extern std::atomic<long long> g_launch_count;
-static inline void counted(int n) { g_launch_count.fetch_add(n, std::memory_order_relaxed); }
+// launches go to the process's count, or, while this thread captures them, to
+// the graph's (they count as they run, hat_loop_count)
+static thread_local long long *t_captured = nullptr;
+static inline void counted(int n)
+{
+    if (t_captured) *t_captured += n;
+    else g_launch_count.fetch_add(n, std::memory_order_relaxed);
+}
 
 // diagonal dr + i di of A at an interior edge: the curl-curl part p sp + q sq
 // (p, q: the weights of the curls beside the edge; sp, sq: the sums of 1 / d of
@@ -973,15 +980,15 @@ static cudaError_t hat_graph_build(HatGraph &hg, cudaGraph_t graph, const KArgs<
     const cudaGraph_t body = np.conditional.phGraph_out[0];
     e = cudaStreamBeginCaptureToGraph(hg.cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
-    const long long c0 = g_launch_count.load();
+    hg.launches = 0;
+    t_captured = &hg.launches;
     for (int it = 0; it < kHatBody; it++) {
         if (ng > 0) launch_hat_iter_multi(args, nrhs, zch, ng, hg.cap);
         else launch_hat_iter(args[0], nrhs[0], hg.cap);
     }
     counted(1);
     kh_more<<<1, 32, 0, hg.cap>>>(p, h);
-    hg.launches = g_launch_count.load() - c0;
-    g_launch_count.fetch_sub(hg.launches);  // counted as they run (hat_loop_count)
+    t_captured = nullptr;
     cudaGraph_t out = nullptr;
     return cudaStreamEndCapture(hg.cap, &out);
 }

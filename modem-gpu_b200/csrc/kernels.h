@@ -12,8 +12,8 @@ namespace mt3d {
 // stream.  Every block of such a kernel calls launch_wait before it touches
 // what earlier kernels read or wrote, also one that has nothing to do, so that
 // a kernel that has ended implies that all before it have.  For iterations that
-// are launched one by one: 175.0 against 167.4 us an FP64 iteration of 64 x 64
-// x 48 cells and 2 right-hand sides.  (Inside the FP32 cycles' graph it took
+// are launched one by one: 167.4 us an FP64 iteration of 64 x 64 x 48 cells and 2
+// right-hand sides, 175.0 launched behind the stream.  (Inside the FP32 cycles' graph it took
 // 1.3 % more time on 200 x 200 x 100 cells, and 18 % more on 24^3 with the next
 // kernel let in at the start of this one.)
 #ifdef __CUDACC__

@@ -705,9 +705,9 @@ int Solver::run_hat(int nrhs, int maxit)
         for (int it = 0; it < maxit; it++) launch_hat_iter(a, nrhs, stream_, next_events(4));
     } else {
         // the cycle as one CUDA graph, replayed while its arguments hold
-        ran_ = &hat_graph_;
         const cudaError_t e = hat_graph_run(hat_graph_, &a, &nrhs, nullptr, 0, maxit, stream_);
         if (e != cudaSuccess) return check(e, "fused BiCGStab graph");
+        ran_ = &hat_graph_;
     }
     launch_bicg_finish(a, nrhs, stream_);
     launch_hat_conv(a, nrhs, stream_);
@@ -721,8 +721,9 @@ int Solver::run_hat_multi(const KArgs<float> *args, const int *nrhs, const int *
             if (launch_hat_iter_multi(args, nrhs, zch, ng, s, fp32_events(4))) return 5;
         return 0;
     }
+    if (hat_graph_run(hat_graph_multi_, args, nrhs, zch, ng, maxit, s) != cudaSuccess) return 4;
     ran_ = &hat_graph_multi_;
-    return hat_graph_run(hat_graph_multi_, args, nrhs, zch, ng, maxit, s) == cudaSuccess ? 0 : 4;
+    return 0;
 }
 
 KArgs<float> Solver::hat_args(int nrhs)

@@ -340,10 +340,10 @@ def stencil_bytes(kprec: int, nE: int, nN: int, fused: bool = False) -> float:
 
 # DRAM bytes (read + write) per edge and right-hand side of one stencil
 # launch, measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum) on
-# the 200x200x100 workload: the unfused kct_vt with 8 right-hand sides, and the
-# fused kh_vt with 2, averaged over the four stages of the polynomial iteration
+# the 200x200x100 model with 8 right-hand sides: the unfused kct_vt, and the fused
+# kh_vt averaged over the four stages of the polynomial iteration
 TRAFFIC_PER_EDGE_RHS = 28.7
-TRAFFIC_PER_EDGE_RHS_FUSED = 23.3
+TRAFFIC_PER_EDGE_RHS_FUSED = 24.0
 
 
 def surface_sites(model: models.Model, nrec: int) -> np.ndarray:

@@ -315,7 +315,10 @@ __global__ void k_bc_coef(BcArgs a, int nslices)
 // rate, were slower: 20.6 to 27.9 ms for the first.)  The error against dense 64-bit solves is the same (2e-14).
 // ---------------------------------------------------------------------------
 constexpr int kBcT = 5;                  // tile edge and panel width
-constexpr int kBcMaxN = 20;              // tiles along a line
+// tiles along a line: 210 threads with a tile each and 4 panel warps, at 168
+// registers, take 59 of an SM's 64 thousand; a longer line would need two tiles a
+// thread or a second SM
+constexpr int kBcMaxN = 20;
 constexpr int kBcMaxM = kBcT * kBcMaxN;  // longest line
 constexpr int kBcOwn = 32 - kBcT;        // columns of a panel per panel warp; the other lanes hold the pivots'
 constexpr int kBcMaxThreads = 352;

@@ -345,8 +345,8 @@ __device__ __forceinline__ float2 hat_curl(float2 p1, float2 p0, float a, float2
 // 30 reads of staged fields, here 21 for two nodes), the diagonal's products
 // formed edge by edge and the potentials behind tests, a launch took on average
 // over the four of an iteration, in us: 40^3, 8 right-hand sides 25.6, now 23.1;
-// 64 x 64 x 48, 8: 61, now 52.5; 100 x 100 x 60, 2: 43.6, now 36.4; 200 x 200 x
-// 100, 1: 111, now 92; 4: 376, now 308.  Of that the plane tables in registers
+// 64 x 64 x 48, 8: 61, now 52.8; 100 x 100 x 60, 2: 43.6, now 36.4; 200 x 200 x
+// 100, 1: 111, now 92; 4: 376, now 311.  Of that the plane tables in registers
 // give 2 % (they fell out of the L1 cache, 28 KB beside the ring, and were
 // waited for on every plane), and the pairs of rows four apart 2 to 3 %.
 template <bool gd, bool has_aux, typename F>

@@ -169,7 +169,8 @@ template <typename K> static int stage_setup(K kern, size_t smem, int slot)
 }
 
 // Time of a launch of c chunks of len planes (the last of them shorter) over
-// `layer` blocks each, in planes of a block that has its SM to itself.  A block
+// `layer` blocks each, in planes of a block that has one of the B200's 148 SMs to
+// itself.  A block
 // costs a plane and a half to start; each further block on an SM slows all of
 // them down by a fifth (the fused FP32 stencil when fitted: 1.55, 1.85, 2.2 and
 // 2.5 us a plane with one to four blocks, so latency counts for more than
@@ -193,8 +194,11 @@ static double stage_time(long layer, int c, int len, int last, long resident)
 // 200 x 200 x 100 cells and 1 to 8 right-hand sides the choice takes 1.9 % more
 // time for the fused FP32 stencil and 1.0 % for the FP64 one (mean; 12 and 7 % at
 // most), and 8 % with half of them left; one count for a single right-hand side
-// in chunks of at least 8 planes took 22.3 instead of 10.9 us a launch on 24^3
-// cells with 2 right-hand sides.
+// in chunks of at least 8 planes took the fused stencil 22.3 instead of 10.9 us a
+// launch on 24^3 cells with 2 right-hand sides.  The unfused FP32 iteration, for
+// which nothing was fitted, takes less time with it (and its launches chained)
+// everywhere: without the grad-div term 74 -> 43 us on 24^3 cells with 2 right-hand sides, 139 -> 126 on
+// 40^3 with 8, 115 -> 97 on 64 x 64 x 48 with 2, 760 -> 733 on 100 x 100 x 60 with 8.
 int stage_chunks(int nz, int tiles, int resident, int nrhs)
 {
     struct Last {
@@ -218,10 +222,12 @@ int stage_chunks(int nz, int tiles, int resident, int nrhs)
 
 template <typename T> static dim3 stage_grid(const KArgs<T> &a, int nrhs, int resident)
 {
-    // without the grad-div term a solve ends with the iteration's own residual
-    // (FWDsolve3D and its divergence correction), which other sums leave a few
-    // per cent from the true one: there the sums keep the order of the count for
-    // one right-hand side in chunks of at least 8 planes
+    // without the grad-div term an FP64 solve ends with the iteration's own
+    // residual, as FWDsolve3D does before a divergence correction, and that lies a
+    // few per cent from the true one, to either side with the order of the sums:
+    // there they keep the order of the count for one right-hand side in chunks of
+    // at least 8 planes (the start of a call and the residual of a mixed cycle with
+    // them, one launch a cycle each)
     int c = 1;
     if (a.zchunks) {
         c = a.zchunks;

@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <type_traits>
 
 #include "kernels.h"
 #include "solver.h"
@@ -77,13 +78,17 @@ __device__ __forceinline__ double rcp_fast(double x)
 }
 // 1 / z for any z: conj(z) / |z|^2 where |z|^2 is far from over- and underflow,
 // as with all but absurd frequencies and cell sizes, Smith's algorithm otherwise
-// (out of line: inlined five times in a panel's sweep it made 40^3 cells 5 % slower;
-// the test itself costs 0 to 2.5 %)
+// (out of line)
+// |z|^2 in 2^-960 .. 2^960 (so not a NaN): by its exponent, off the FP64 pipe
+__device__ __forceinline__ bool square_ok(double n)
+{
+    return (unsigned)__double2hiint(n) - ((1023u - 960u) << 20) < (2u * 960u) << 20;
+}
 __device__ __noinline__ double2 crcp_far(double2 z) { return cdv(c2(1.0, 0.0), z); }
 __device__ __forceinline__ double2 crcp(double2 z)
 {
     const double n = fma(z.x, z.x, z.y * z.y);
-    if (!(n > 1e-290 && n < 1e290)) return crcp_far(z);
+    if (!square_ok(n)) return crcp_far(z);
     const double iv = rcp_fast(n);
     return c2(z.x * iv, -z.y * iv);
 }
@@ -309,8 +314,8 @@ __global__ void k_bc_coef(BcArgs a, int nslices)
 // Bound by FP64 arithmetic for long lines (half of m^3 complex multiply-adds
 // a line) and by the panels' chains for short ones.  One polarisation, against
 // the band elimination of k_bc2d (a pivot at a time, two block barriers and
-// the whole window through shared memory for each): 200 x 200 x 100 cells 18.7
-// against 208.4 ms, 101 x 83 x 61 1.69 against 17.8 ms, 40^3 0.38 against
+// the whole window through shared memory for each): 200 x 200 x 100 cells 18.4
+// against 208.4 ms, 101 x 83 x 61 1.67 against 17.8 ms, 40^3 0.38 against
 // 4.66 ms.  (8 x 8 blocks in FP64 matrix instructions, which run at the same
 // rate, were slower: 20.6 to 27.9 ms for the first.)  The error against dense 64-bit solves is the same (2e-14).
 // ---------------------------------------------------------------------------
@@ -429,7 +434,12 @@ template <bool mid, int threads, int blocks> __global__ void __launch_bounds__(t
         // R and G of panel k from the published entries, panel k - 1 applied first
         const int own = pw * kBcOwn + lane;
         const bool dup = lane >= kBcOwn, ok = dup || own <= MP;
-        auto sweep = [&](int k) {
+        // far: pivots inverted without squares where those over- or underflow.
+        // Otherwise false when one did, in all lanes and warps alike; nothing that a
+        // second go reads has changed then.  A test and a branch at every pivot
+        // made 200 x 200 x 100 cells 2.2 % slower than none, the tests alone and a
+        // branch a panel 1.3 %
+        auto sweep_as = [&](int k, auto far) {
             const int P = k * T, K = P - T, col = dup ? P + lane - kBcOwn : own;
             const double2 *R = Rb + ((k - 1) & 1) * T * MA, *G = Gb + ((k - 1) & 1) * T * MA;
             double2 *Rn = Rb + (k & 1) * T * MA, *Gn = Gb + (k & 1) * T * MA;
@@ -453,12 +463,20 @@ template <bool mid, int threads, int blocks> __global__ void __launch_bounds__(t
             if (!dup && ok)
 #pragma unroll
                 for (int r = 0; r < T; r++) Rn[r * MA + col] = v[r];
+            bool ok_sq = true;
 #pragma unroll
             for (int p = 0; p < T; p++) {
                 double2 l[T];
 #pragma unroll
                 for (int r = 0; r < T; r++) l[r] = shfl2(v[r], kBcOwn + p);
-                const double2 iv = crcp(l[p]);
+                double2 iv;
+                if constexpr (far.value) {
+                    iv = crcp(l[p]);
+                } else {
+                    const double n2 = fma(l[p].x, l[p].x, l[p].y * l[p].y), den = rcp_fast(n2);
+                    iv = c2(l[p].x * den, -l[p].y * den);
+                    ok_sq = ok_sq && square_ok(n2);
+                }
                 const bool pc = col == P + p;
                 const double2 g = pc ? iv : cm(v[p], iv);
 #pragma unroll
@@ -472,6 +490,10 @@ template <bool mid, int threads, int blocks> __global__ void __launch_bounds__(t
             if (!dup && ok)
 #pragma unroll
                 for (int r = 0; r < T; r++) Gn[r * MA + col] = v[r];
+            return ok_sq;
+        };
+        auto sweep = [&](int k) {
+            if (!sweep_as(k, std::false_type{})) sweep_as(k, std::true_type{});
         };
         for (int st = 0; st < steps; st++) {
             const bool more = st + 1 < steps;
